@@ -9,6 +9,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
@@ -18,9 +19,9 @@ LIB = os.path.join(HERE, "libfluamsl.so")
 EXE = os.path.join(HERE, "fluam")
 
 CU_SOURCES = ["fsl_particles.cu", "fsl_fft.cu", "fsl_group.cu", "fsl_api.cu", "fsl_batch.cu", "fsl_server.cu", "fsl_noalloc.cu",
-              "fsl_fp64.cu", "fsl_q2d.cu", "fsl_inc.cu"]
+              "fsl_fp64.cu", "fsl_fft_g.cu", "fsl_q2d.cu", "fsl_inc.cu"]
 CPP_SOURCES = ["fsl_datamain.cpp"]
-HEADERS = ["fsl_internal.cuh", "fsl_group.cuh", "fsl_fft_reg.cuh", "fsl_fft_lines.cuh"]
+HEADERS = ["fsl_internal.cuh", "fsl_group.cuh", "fsl_fft_reg.cuh", "fsl_fft_lines.cuh", "fsl_fft_v.cuh", "fsl_bulk.cuh"]
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -44,7 +45,7 @@ def _stale(target, deps):
 def build(force=False, verbose=False, ptxas_info=False):
     os.makedirs(BUILD, exist_ok=True)
     hdrs = [os.path.join(CSRC, h) for h in HEADERS] + [os.path.join(ROOT, "include", "fluamsl.h")]
-    objs = []
+    objs, cmds = [], []
     for src in CU_SOURCES + CPP_SOURCES:
         path = os.path.join(CSRC, src)
         obj = os.path.join(BUILD, src + ".o")
@@ -58,7 +59,11 @@ def build(force=False, verbose=False, ptxas_info=False):
             cmd = [nvcc()] + flags + ["-c", path, "-o", obj]
             if verbose:
                 print(" ".join(cmd))
-            subprocess.run(cmd, check=True)
+            cmds.append(cmd)
+    # the sources compile independently of each other
+    with ThreadPoolExecutor(max(1, min(len(cmds), os.cpu_count() or 1))) as pool:
+        for r in [pool.submit(subprocess.run, c, check=True) for c in cmds]:
+            r.result()
     if force or _stale(LIB, objs):
         tmp = LIB + ".tmp"
         subprocess.run([nvcc()] + ARCH + ["-shared", "-o", tmp] + objs + ["-lcudart"], check=True)

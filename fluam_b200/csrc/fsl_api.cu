@@ -274,10 +274,11 @@ int fsl_set_velocity_f64(fsl_handle* h, const double* in) {
   FSL_TRY(cudaMemcpyAsync(rep(h).v64, in, sizeof(double) * 3 * (size_t)params(h).nc,
                           cudaMemcpyHostToDevice, s));
   // src/runSchemeIncompressible.cu:82-96: the projection of the initial field
+  const fsl::GPlan* gp = fsl::fft_general(h->group.fft);
   fsl::launch_inc_load(B, s);
-  fsl::launch_fft64_3d(B, -1, 0, s);
-  fsl::launch_inc_fourier(B, 0, s);
-  fsl::launch_fft64_3d(B, +1, 1, s);
+  fsl::launch_g_forward(B, gp, 3, s);
+  fsl::launch_g_z(B, gp, 2, s);
+  fsl::launch_g_inverse(B, gp, 3, 0, 1.0, s);
   if ((rc = check_launch())) return rc;
   FSL_TRY(cudaStreamSynchronize(s));
   return FSL_OK;

@@ -4,11 +4,10 @@
 // noise (Box-Muller in FP64 on the same Philox words), spreading with FP64
 // atomics, W, the FFT-based Stokes solve and the interpolation.  fluam itself
 // is FP64 throughout, so this form carries the reference's own arithmetic on
-// the GPU; it is the third form of the precision study and is written for
-// clarity over speed: one thread per particle and component for the particle
-// side, shared-memory Stockham lines (any 2,3,5,7,11-smooth length) with the
-// twiddles evaluated in place for the FFTs.  The cell list and the forces
-// are the shared FP64 kernels of fsl_particles.cu.
+// the GPU; it is the third form of the precision study.  One thread per
+// particle and component for the particle side; the transforms are those of
+// fsl_fft_g.cu, the cell list and the forces the shared FP64 kernels of
+// fsl_particles.cu.
 #include "fsl_internal.cuh"
 
 namespace fsl {
@@ -173,8 +172,8 @@ __global__ void k_spread64(FSL_KARGS, int drift) {
 
 // ------------------------------------------------------------------- W ---
 // W = f / dV + nfac div(Sigma) per cell (the formulas of k_wbuild in FP64),
-// written as the real part of the spectrum buffer; the spread field is
-// cleared behind the read.
+// into the transform's real field; the spread field is cleared behind the
+// read.
 template <bool ONE>
 __global__ void k_wbuild64(FSL_KARGS, int nsets, double nfac) {
   FSL_REP_AT(blockIdx.y);
@@ -207,223 +206,9 @@ __global__ void k_wbuild64(FSL_KARGS, int nsets, double nfac) {
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      R.z64[c * nc + i] = make_double2(w[c], 0.0);
+      R.w64[c * nc + i] = w[c];
       g[c * nc + i] = 0.0;
     }
-  }
-}
-
-// ------------------------------------------------------------------- FFT ---
-// Complex lines of length n along one axis of the three-component array,
-// transformed in shared memory by the Stockham autosort algorithm
-// (Govindaraju et al., SC'08) with mixed radices 4, 2, 3, 5, 7, 11: stage
-// with radix p and span Ns reads v_r = X[j + r n/p], twiddles v_r by
-// exp(dir 2 pi i r (j mod Ns) / (Ns p)), a p-point DFT, and writes
-// Y[(j / Ns) Ns p + (j mod Ns) + r Ns].  Unnormalised, dir -1 forward.
-struct Radix64 {
-  int n, nf, f[12];
-};
-
-Radix64 radices(int n) {
-  Radix64 R{};
-  R.n = n;
-  while (n % 4 == 0) { R.f[R.nf++] = 4; n /= 4; }
-  const int ps[5] = {2, 3, 5, 7, 11};
-  for (int p : ps)
-    while (n % p == 0) { R.f[R.nf++] = p; n /= p; }
-  return R;
-}
-
-template <int Pr>
-__device__ __forceinline__ void dft64(double2 (&v)[Pr], int dir) {
-  if constexpr (Pr == 2) {
-    double2 a = v[0], b = v[1];
-    v[0] = make_double2(a.x + b.x, a.y + b.y);
-    v[1] = make_double2(a.x - b.x, a.y - b.y);
-  } else if constexpr (Pr == 4) {
-    const double2 a0 = make_double2(v[0].x + v[2].x, v[0].y + v[2].y);
-    const double2 a1 = make_double2(v[0].x - v[2].x, v[0].y - v[2].y);
-    const double2 b0 = make_double2(v[1].x + v[3].x, v[1].y + v[3].y);
-    const double2 b1 = make_double2(v[1].x - v[3].x, v[1].y - v[3].y);
-    // multiply b1 by dir * i
-    const double2 ib1 = make_double2(-dir * b1.y, dir * b1.x);
-    v[0] = make_double2(a0.x + b0.x, a0.y + b0.y);
-    v[2] = make_double2(a0.x - b0.x, a0.y - b0.y);
-    v[1] = make_double2(a1.x + ib1.x, a1.y + ib1.y);
-    v[3] = make_double2(a1.x - ib1.x, a1.y - ib1.y);
-  } else {
-    double2 w[Pr], o[Pr];  // w[k] = exp(dir 2 pi i k / Pr)
-#pragma unroll
-    for (int k = 0; k < Pr; ++k) sincospi((double)(2 * k) / Pr * dir, &w[k].y, &w[k].x);
-#pragma unroll
-    for (int q = 0; q < Pr; ++q) {
-      double sx = 0.0, sy = 0.0;
-#pragma unroll
-      for (int r = 0; r < Pr; ++r) {
-        const double2 t = w[(r * q) % Pr];
-        sx += v[r].x * t.x - v[r].y * t.y;
-        sy += v[r].x * t.y + v[r].y * t.x;
-      }
-      o[q] = make_double2(sx, sy);
-    }
-#pragma unroll
-    for (int q = 0; q < Pr; ++q) v[q] = o[q];
-  }
-}
-
-template <int Pr>
-__device__ void stage64(const double2* __restrict__ X, double2* __restrict__ Y, int n, int Ns,
-                        int nl, int dir) {
-  const int nb = n / Pr;
-  for (int t = threadIdx.x; t < nl * nb; t += blockDim.x) {
-    const int l = t / nb, j = t - l * nb;
-    const double2* x = X + (size_t)l * n;
-    double2* y = Y + (size_t)l * n;
-    const int k = j % Ns;
-    double2 v[Pr];
-#pragma unroll
-    for (int r = 0; r < Pr; ++r) v[r] = x[j + r * nb];
-    if (Ns > 1) {
-#pragma unroll
-      for (int r = 1; r < Pr; ++r) {
-        double s, c;
-        sincospi((double)(2 * r * k) / (double)(Ns * Pr) * dir, &s, &c);
-        v[r] = make_double2(v[r].x * c - v[r].y * s, v[r].x * s + v[r].y * c);
-      }
-    }
-    dft64<Pr>(v, dir);
-    const int d = (j / Ns) * Ns * Pr + k;
-#pragma unroll
-    for (int r = 0; r < Pr; ++r) y[d + r * Ns] = v[r];
-  }
-}
-
-constexpr int kF64Threads = 256;
-constexpr int kF64Elems = 1024;  // lines x length per block: 2 x 16 KB buffers
-
-// Lines of one block: axis 0 takes nl consecutive rows (contiguous);
-// axes 1 and 2 take nl consecutive x at one (comp, other index), element
-// stride mx or mx my; ncomp field components.  to_real: the last inverse
-// pass stores Re / nc to v64.
-template <bool ONE>
-__global__ void __launch_bounds__(kF64Threads) k_fft64(FSL_KARGS, int axis, const Radix64 rad,
-                                                       int dir, int to_real, int ncomp) {
-  FSL_REP_AT(blockIdx.y);
-  __shared__ double2 sA[kF64Elems], sB[kF64Elems];
-  const int n = rad.n;
-  const int mx = P.mx, my = P.my, mz = P.mz;
-  const size_t nc = (size_t)P.nc;
-  const int nl = kF64Elems / n < 1 ? 1 : (kF64Elems / n > 32 ? 32 : kF64Elems / n);
-  size_t base;
-  size_t estride, lstride;
-  int nvalid;
-  if (axis == 0) {
-    const long nrows = (long)ncomp * my * mz;
-    const long r0 = (long)blockIdx.x * nl;
-    if (r0 >= nrows) return;
-    base = (size_t)r0 * mx;
-    estride = 1;
-    lstride = (size_t)mx;
-    nvalid = (int)min((long)nl, nrows - r0);
-  } else {
-    const int gx = (mx + nl - 1) / nl;
-    const int other = axis == 1 ? mz : my;
-    const long b = blockIdx.x;
-    if (b >= (long)ncomp * other * gx) return;
-    const int xg = (int)(b % gx);
-    const long rest = b / gx;
-    const int o = (int)(rest % other), comp = (int)(rest / other);
-    const int x0 = xg * nl;
-    base = comp * nc + x0 + (axis == 1 ? (size_t)mx * my * o : (size_t)mx * o);
-    estride = axis == 1 ? (size_t)mx : (size_t)mx * my;
-    lstride = 1;
-    nvalid = min(nl, mx - x0);
-  }
-  double2* Z = R.z64;
-  // load: consecutive threads take consecutive addresses
-  for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
-    int l, j;
-    if (axis == 0) { l = t / n; j = t - l * n; }
-    else { j = t / nl; l = t - j * nl; }
-    sA[l * n + j] = l < nvalid ? Z[base + l * lstride + j * estride] : make_double2(0.0, 0.0);
-  }
-  __syncthreads();
-  double2* X = sA;
-  double2* Y = sB;
-  int Ns = 1;
-  for (int s = 0; s < rad.nf; ++s) {
-    const int p = rad.f[s];
-    switch (p) {
-      case 4: stage64<4>(X, Y, n, Ns, nl, dir); break;
-      case 2: stage64<2>(X, Y, n, Ns, nl, dir); break;
-      case 3: stage64<3>(X, Y, n, Ns, nl, dir); break;
-      case 5: stage64<5>(X, Y, n, Ns, nl, dir); break;
-      case 7: stage64<7>(X, Y, n, Ns, nl, dir); break;
-      default: stage64<11>(X, Y, n, Ns, nl, dir); break;
-    }
-    __syncthreads();
-    double2* tmp = X;
-    X = Y;
-    Y = tmp;
-    Ns *= p;
-  }
-  const double inv_nc = 1.0 / (double)nc;
-  for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
-    int l, j;
-    if (axis == 0) { l = t / n; j = t - l * n; }
-    else { j = t / nl; l = t - j * nl; }
-    if (l >= nvalid) continue;
-    const size_t a = base + l * lstride + j * estride;
-    if (to_real) R.v64[a] = X[l * n + j].x * inv_nc;
-    else Z[a] = X[l * n + j];
-  }
-}
-
-// Fourier-space solve per mode (src/stokesLimitFunctions.cu:2399-2451 with
-// the staggered shifts of src/realToComplex.cu:263-303 and the tables of
-// src/initializePrefactorFourierSpace.cu:39-69, evaluated in place).
-template <bool ONE>
-__global__ void k_solve64(FSL_KARGS) {
-  FSL_REP_AT(blockIdx.y);
-  const int mx = P.mx, my = P.my, mz = P.mz;
-  const size_t nc = (size_t)P.nc;
-  const double pi = 3.141592653589793238462643383280;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nc;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(i % mx), r = (int)(i / mx);
-    const int ky = r % my, kz = r / my;
-    const int kk[3] = {kx, ky, kz};
-    const int m[3] = {mx, my, mz};
-    const double invd[3] = {P.invdx, P.invdy, P.invdz};
-    double c[3], sn[3], gk[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double arg = pi * kk[a] / (double)m[a];
-      sincos(arg, &sn[a], &c[a]);
-      gk[a] = 2 * invd[a] * sn[a];
-    }
-    double2 W[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double2 z = R.z64[a * nc + i];
-      // shift -1: W (cos - i sin)
-      W[a] = make_double2(z.x * c[a] + z.y * sn[a], z.y * c[a] - z.x * sn[a]);
-    }
-    double2 V[3];
-    if (i == 0) {
-      V[0] = V[1] = V[2] = make_double2(0.0, 0.0);
-    } else {
-      const double L = -(gk[0] * gk[0]) - (gk[1] * gk[1]) - (gk[2] * gk[2]);
-      const double den = -P.eta * L;
-      const double GWr = gk[0] * W[0].x + gk[1] * W[1].x + gk[2] * W[2].x;
-      const double GWi = gk[0] * W[0].y + gk[1] * W[1].y + gk[2] * W[2].y;
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        V[a] = make_double2((W[a].x + gk[a] * GWr / L) / den, (W[a].y + gk[a] * GWi / L) / den);
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)  // shift +1: V (cos + i sin)
-      R.z64[a * nc + i] = make_double2(V[a].x * c[a] - V[a].y * sn[a], V[a].y * c[a] + V[a].x * sn[a]);
   }
 }
 
@@ -502,32 +287,7 @@ void launch_interp_update64(const Batch& B, int stage, cudaStream_t s) {
     FSL_GO_T(k_interp_update64, 3, g, kPartThreads, 0, s, B, stage);
 }
 
-// The line passes of a forward (dir -1: x, y[, z]) or inverse (dir +1:
-// [z,] y, x, the x pass storing Re / nc) transform of ncomp components over
-// the first naxes axes.
-static void fft64_passes(const Batch& B, int ncomp, int naxes, int dir, cudaStream_t s,
-                         int to_real = 1) {
-  const int m[3] = {B.mx, B.my, B.mz};
-  Radix64 rad[3];
-  unsigned gb[3];
-  for (int a = 0; a < naxes; ++a) {
-    rad[a] = radices(m[a]);
-    const int n = m[a];
-    const int nl = kF64Elems / n < 1 ? 1 : (kF64Elems / n > 32 ? 32 : kF64Elems / n);
-    if (a == 0) gb[a] = (unsigned)(((long)ncomp * B.my * B.mz + nl - 1) / nl);
-    else gb[a] = (unsigned)((long)ncomp * (a == 1 ? B.mz : B.my) * ((B.mx + nl - 1) / nl));
-  }
-  if (dir < 0) {
-    for (int a = 0; a < naxes; ++a)
-      FSL_GO(k_fft64, dim3(gb[a], B.nrep), kF64Threads, 0, s, B, a, rad[a], -1, 0, ncomp);
-  } else {
-    for (int a = naxes - 1; a >= 0; --a)
-      FSL_GO(k_fft64, dim3(gb[a], B.nrep), kF64Threads, 0, s, B, a, rad[a], +1, a == 0 ? to_real : 0,
-             ncomp);
-  }
-}
-
-void launch_solve64(const Batch& B, int nsets, double nfac, cudaStream_t s, Prof* prof) {
+void launch_solve64(const Batch& B, const GPlan* g, int nsets, double nfac, cudaStream_t s, Prof* prof) {
   const int tb = 256;
   unsigned bc = blocks_for((long)B.nc, tb);
   const unsigned cap = (unsigned)((148 * 16 + B.nrep - 1) / B.nrep);
@@ -535,18 +295,12 @@ void launch_solve64(const Batch& B, int nsets, double nfac, cudaStream_t s, Prof
   if (prof) prof->mark(s, "wbuild64");
   FSL_GO(k_wbuild64, dim3(bc, B.nrep), tb, 0, s, B, nsets, nfac);
   if (prof) prof->mark(s, "fft64");
-  fft64_passes(B, 3, 3, -1, s);
+  int n = launch_g_forward(B, g, 3, s);
   if (prof) prof->mark(s, "solve64");
-  FSL_GO(k_solve64, dim3(bc, B.nrep), tb, 0, s, B);
+  launch_g_z(B, g, 0, s);
   if (prof) prof->mark(s, "fft64");
-  fft64_passes(B, 3, 3, +1, s);
-  if (prof) prof->count(1 + 3 + 1 + 3);
-}
-
-void launch_fft64_2d(const Batch& B, int dir, cudaStream_t s) { fft64_passes(B, 2, 2, dir, s); }
-
-void launch_fft64_3d(const Batch& B, int dir, int to_real, cudaStream_t s) {
-  fft64_passes(B, 3, 3, dir, s, to_real);
+  n += launch_g_inverse(B, g, 3, 0, 1.0, s);
+  if (prof) prof->count(2 + n);
 }
 
 }  // namespace fsl

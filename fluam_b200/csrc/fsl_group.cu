@@ -26,7 +26,7 @@ size_t align_up(size_t n) { return (n + kAlign - 1) / kAlign * kAlign; }
 // Byte offsets of one slot's buffers inside its arena.
 struct SlotLayout {
   size_t q, qp, F, u, qw, ws, cell_of, tmp, sorted, bpp_cnt, bpp_off, bfp_cnt, bfp_off, cnt, fill, start,
-      bsum, ljtab, noise, ndiv, stc, grid, spec, v, wbuf, noise64, v64, z64, err, t, q0, obs, obs_part, obs_ticket,
+      bsum, ljtab, noise, ndiv, stc, grid, spec, v, wbuf, noise64, v64, z64, w64, err, t, q0, obs, obs_part, obs_ticket,
       start1, sorted1, ws1, vl_cnt, vl_idx, qref, vl_flag, bar, total;
 };
 
@@ -76,7 +76,8 @@ SlotLayout layout(const Params& P, int np_cap) {
   L.wbuf = take(f64 ? 0 : sizeof(float) * 3 * nc);
   L.noise64 = take(f64 ? sizeof(double) * noise : 0);
   L.v64 = take(f64 ? sizeof(double) * 3 * nc : 0);
-  L.z64 = take(f64 ? sizeof(double2) * 3 * nc : 0);
+  L.z64 = take(f64 ? sizeof(double2) * 3 * (size_t)P.my * P.mz * P.mxh : 0);
+  L.w64 = take(f64 ? sizeof(double) * 3 * nc : 0);
   L.err = take(sizeof(int) * 4);
   L.t = take(sizeof(uint64_t));
   L.q0 = take(P.observe ? sizeof(double) * 3 * np : 0);
@@ -361,6 +362,7 @@ int slot_alloc(Slot& s, const Params& P, int np_cap, cudaStream_t st) {
   r.noise64 = f64 ? (double*)(base + L.noise64) : nullptr;
   r.v64 = f64 ? (double*)(base + L.v64) : nullptr;
   r.z64 = f64 ? (double2*)(base + L.z64) : nullptr;
+  r.w64 = f64 ? (double*)(base + L.w64) : nullptr;
   r.err = (int*)(base + L.err);
   r.t = (uint64_t*)(base + L.t);
   r.q0 = P.observe ? (double*)(base + L.q0) : nullptr;
@@ -838,19 +840,19 @@ void group_enqueue_step(Group& g) {
     // the advection of the second taken from the prediction
     join_noise();
     pr.mark(s, "inc_substep1");
+    const GPlan* gp = fft_general(g.fft);
     launch_inc_w(B, 0, s);
-    launch_fft64_3d(B, -1, 0, s);
-    launch_inc_fourier(B, 1, s);
-    launch_fft64_3d(B, +1, 0, s);
-    launch_inc_pred(B, s);
+    int nl = launch_g_forward(B, gp, 3, s);
+    launch_g_z(B, gp, 1, s);
+    nl += launch_g_inverse(B, gp, 3, 1, 1.0, s);  // the prediction (v + u) / 2
     chk("substep 1");
     pr.mark(s, "inc_substep2");
     launch_inc_w(B, 1, s);
-    launch_fft64_3d(B, -1, 0, s);
-    launch_inc_fourier(B, 1, s);
-    launch_fft64_3d(B, +1, 1, s);
+    nl += launch_g_forward(B, gp, 3, s);
+    launch_g_z(B, gp, 1, s);
+    nl += launch_g_inverse(B, gp, 3, 0, 1.0, s);
     chk("substep 2");
-    pr.count(2 * (1 + 3 + 1 + 3) + 1);
+    pr.count(4 + nl);
     pr.mark(s, "counter");
     launch_step_counter(B, s);
     chk("counter");
@@ -873,9 +875,8 @@ void group_enqueue_step(Group& g) {
     launch_q2_field(B, s, &pr);
     chk("spread");
     pr.count(2 + pk);
-    launch_q2_solve(B, s, &pr);
+    launch_q2_solve(B, fft_general(g.fft), s, &pr);
     chk("solve");
-    pr.count(2 + 1 + 2);
     pr.mark(s, "q2_update");
     launch_q2_update(B, 1, s);
     launch_q2_update(B, 2, s);

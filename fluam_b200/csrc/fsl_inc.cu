@@ -5,9 +5,10 @@
 // Crank-Nicolson viscous term and a midpoint advection in two substeps that
 // share one noise draw, each substep a W build in real space, a forward FFT,
 // the shifted Crank-Nicolson solve with the divergence-free projection per
-// mode, and an inverse FFT.  The prediction u^{n+1/2} of the first substep
-// lives in the 8-byte spread buffer (Rep::grid, unused by this scheme).  The
-// FFT passes are those of the FP64 form (fsl_fp64.cu).
+// mode, and an inverse FFT.  The prediction u^{n+1/2} = (v + u^n) / 2 of the
+// first substep (src/realToComplex.cu:108-119), written by the inverse
+// transform, lives in the 8-byte spread buffer (Rep::grid, unused by this
+// scheme).  The transforms and the solve are those of fsl_fft_g.cu.
 #include "fsl_internal.cuh"
 
 namespace fsl {
@@ -96,79 +97,19 @@ __global__ void k_inc_w(FSL_KARGS, int second) {
     wy -= idz * f4 * Rn[v0 + 4 * n];
     wz -= idx * f4 * Rn[v2 + 2 * n];
     wz -= idy * f4 * Rn[v1 + 4 * n];
-    R.z64[i] = make_double2(wx, 0.0);
-    R.z64[n + i] = make_double2(wy, 0.0);
-    R.z64[2 * n + i] = make_double2(wz, 0.0);
+    R.w64[i] = wx;
+    R.w64[n + i] = wy;
+    R.w64[2 * n + i] = wz;
   }
 }
 
-// Per mode: shift(-1), the Crank-Nicolson solve with the projection
-// (src/kernelUpdateVIncompressible.cu:20-73) or the projection alone
-// (src/projectionDivergenceFree.cu:21-90), shift(+1); the tables of
-// src/initializePrefactorFourierSpace.cu:39-69 evaluated in place.
-template <bool ONE>
-__global__ void k_inc_fourier(FSL_KARGS, int solve) {
-  FSL_REP_AT(blockIdx.y);
-  const int mx = P.mx, my = P.my, mz = P.mz;
-  const size_t nc = (size_t)P.nc;
-  const double pi = 3.141592653589793238462643383280;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nc;
-       i += (size_t)gridDim.x * blockDim.x) {
-    const int kx = (int)(i % mx), r = (int)(i / mx);
-    const int ky = r % my, kz = r / my;
-    const int kk[3] = {kx, ky, kz};
-    const int m[3] = {mx, my, mz};
-    const double invd[3] = {P.invdx, P.invdy, P.invdz};
-    double c[3], sn[3], g[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      sincos(pi * kk[a] / (double)m[a], &sn[a], &c[a]);
-      g[a] = 2 * invd[a] * sn[a];
-    }
-    double2 W[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      const double2 zz = R.z64[a * nc + i];
-      W[a] = make_double2(zz.x * c[a] + zz.y * sn[a], zz.y * c[a] - zz.x * sn[a]);
-    }
-    double2 V[3] = {W[0], W[1], W[2]};
-    if (i != 0) {
-      const double GG = -(g[0] * g[0]) - (g[1] * g[1]) - (g[2] * g[2]);
-      const double GWr = g[0] * W[0].x + g[1] * W[1].x + g[2] * W[2].x;
-      const double GWi = g[0] * W[0].y + g[1] * W[1].y + g[2] * W[2].y;
-      const double den = solve ? 1 - 0.5 * P.dt * P.eta * GG / P.rho : 1.0;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        if (solve)
-          V[a] = make_double2((W[a].x + g[a] * GWr / GG) / den, (W[a].y + g[a] * GWi / GG) / den);
-        else
-          V[a] = make_double2(W[a].x + g[a] * GWr / GG, W[a].y + g[a] * GWi / GG);
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-      R.z64[a * nc + i] = make_double2(V[a].x * c[a] - V[a].y * sn[a], V[a].y * c[a] + V[a].x * sn[a]);
-  }
-}
-
-// u^{n+1/2} = (Re(Z) / nc + u^n) / 2 into the spread buffer
-// (src/realToComplex.cu:108-119)
-template <bool ONE>
-__global__ void k_inc_pred(FSL_KARGS) {
-  FSL_REP_AT(blockIdx.y);
-  const size_t n3 = 3 * (size_t)P.nc;
-  double* pred = reinterpret_cast<double*>(R.grid);
-  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n3; k += (size_t)gridDim.x * blockDim.x)
-    pred[k] = 0.5 * ((R.z64[k].x / double(P.nc)) + R.v64[k]);
-}
-
-// Z = u (src/realToComplex.cu:21-38)
+// The transform's real field = u (src/realToComplex.cu:21-38)
 template <bool ONE>
 __global__ void k_inc_load(FSL_KARGS) {
   FSL_REP_AT(blockIdx.y);
   const size_t n3 = 3 * (size_t)P.nc;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n3; k += (size_t)gridDim.x * blockDim.x)
-    R.z64[k] = make_double2(R.v64[k], 0.0);
+    R.w64[k] = R.v64[k];
 }
 
 unsigned cell_blocks(const Batch& B, long work) {
@@ -181,14 +122,6 @@ unsigned cell_blocks(const Batch& B, long work) {
 
 void launch_inc_w(const Batch& B, int second, cudaStream_t s) {
   FSL_GO(k_inc_w, dim3(cell_blocks(B, B.nc), B.nrep), 256, 0, s, B, second);
-}
-
-void launch_inc_fourier(const Batch& B, int solve, cudaStream_t s) {
-  FSL_GO(k_inc_fourier, dim3(cell_blocks(B, B.nc), B.nrep), 256, 0, s, B, solve);
-}
-
-void launch_inc_pred(const Batch& B, cudaStream_t s) {
-  FSL_GO(k_inc_pred, dim3(cell_blocks(B, 3L * B.nc), B.nrep), 256, 0, s, B);
 }
 
 void launch_inc_load(const Batch& B, cudaStream_t s) {

@@ -471,10 +471,12 @@ struct Rep {
   int* start1;
   int* sorted1;
   double* ws1;
-  // FP64 form only (null otherwise): noise, field, complex spectrum
+  // FP64 form only (null otherwise): noise, field, half spectrum
+  // [comp][z][ky][kx], and the real field that a transform starts from
   double* noise64;
   double* v64;
   double2* z64;
+  double* w64;
   int* err;
   uint64_t* t;
   // observables: reference positions q0 [3][np], accumulators (kObsSlots
@@ -765,24 +767,33 @@ void launch_observe(const Batch& B, cudaStream_t s);
 void launch_noise64(const Batch& B, cudaStream_t s);
 void launch_spread64(const Batch& B, int drift, cudaStream_t s);
 void launch_interp_update64(const Batch& B, int stage, cudaStream_t s);
-void launch_solve64(const Batch& B, int nsets, double nfac, cudaStream_t s, Prof* prof);
-// 2-D transforms of two FP64 components (the quasi-2D family)
-void launch_fft64_2d(const Batch& B, int dir, cudaStream_t s);
-// 3-D transforms of three FP64 components; to_real: the inverse's last pass
-// stores Re / nc to Rep::v64 instead of the spectrum
-void launch_fft64_3d(const Batch& B, int dir, int to_real, cudaStream_t s);
+struct GPlan;
+void launch_solve64(const Batch& B, const GPlan* g, int nsets, double nfac, cudaStream_t s, Prof* prof);
 // The incompressible scheme (fsl_inc.cu)
 void launch_inc_w(const Batch& B, int second, cudaStream_t s);
-void launch_inc_fourier(const Batch& B, int solve, cudaStream_t s);
-void launch_inc_pred(const Batch& B, cudaStream_t s);
 void launch_inc_load(const Batch& B, cudaStream_t s);
 // The quasi-2D family (fsl_q2d.cu)
 void launch_q2_forces(const Batch& B, cudaStream_t s);
 void launch_q2_field(const Batch& B, cudaStream_t s, Prof* prof);
-void launch_q2_solve(const Batch& B, cudaStream_t s, Prof* prof);
+void launch_q2_solve(const Batch& B, const GPlan* g, cudaStream_t s, Prof* prof);
 void launch_q2_update(const Batch& B, int stage, cudaStream_t s);
 
+// Transforms of any 2,3,5,7,11-smooth extents (fsl_fft_g.cu), in the
+// precision of the class: the real field (Rep::wbuf or w64) of ncomp
+// components into the half spectrum (spec or z64); the z lines of three
+// components with the solve of every mode (0 Stokes, 1 Crank-Nicolson with
+// projection, 2 projection alone; times 1/nc); the half spectrum back into
+// scale times the real field (v or v64), with pred: (that + v64) / 2 into
+// Rep::grid.  Forward and inverse return the kernels they launched.
+GPlan* gplan_create(const Params& P);
+void gplan_destroy(GPlan* g);
+int launch_g_forward(const Batch& B, const GPlan* g, int ncomp, cudaStream_t s);
+void launch_g_z(const Batch& B, const GPlan* g, int solve, cudaStream_t s);
+int launch_g_inverse(const Batch& B, const GPlan* g, int ncomp, int pred, double scale, cudaStream_t s);
+
 struct FftPlan;  // defined in fsl_fft.cu
+// the plan's general transforms (null where compiled passes serve the class)
+const GPlan* fft_general(const FftPlan* fp);
 FftPlan* fft_plan_create(const Params& P);
 void fft_plan_destroy(FftPlan* fp);
 // Picks the fastest z-pass tile of the plan's candidates, the fastest

@@ -7,11 +7,11 @@
 // around the node at or below it (w = kernelWidth).  One step: noise, the
 // 2-D cell list and forces (only with computeNonBondedForces, as the
 // reference), force and thermal-drift spreading with FP64 atomics into the
-// real parts of the complex field, the optional shear forcing, a 2-D FFT,
+// field, the optional shear forcing, a 2-D FFT,
 // the Fourier-space mobility plus stochastic velocity per mode, the inverse
 // FFT and the particle update (forward Euler or the predictor-corrector on
-// the same velocity field).  The FFT passes are those of the FP64 form
-// (fsl_fp64.cu); the cell list is the shared counting sort (one z layer).
+// the same velocity field).  The transforms are those of fsl_fft_g.cu; the
+// cell list is the shared counting sort (one z layer).
 #include "fsl_internal.cuh"
 
 namespace fsl {
@@ -133,12 +133,12 @@ __global__ void k_q2_zero(FSL_KARGS) {
   FSL_REP_AT(blockIdx.y);
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < 2 * (size_t)P.nc;
        i += (size_t)gridDim.x * blockDim.x)
-    R.z64[i] = make_double2(0.0, 0.0);
+    R.w64[i] = 0.0;
 }
 
 // One thread per particle: g(r) F (with the forces) and the thermal drift
 // -g(r) (kT / var) (r - x_node) (src/quasi2DFunctions.cu:243-281, 287-391)
-// into the real parts of the two field components.
+// into the two field components.
 template <bool ONE>
 __global__ void k_q2_spread(FSL_KARGS) {
   FSL_REP_FLAT(KIND_T1);
@@ -152,8 +152,8 @@ __global__ void k_q2_spread(FSL_KARGS) {
   const int mx = P.mx, my = P.my, w = P.q2_kw;
   const int kx = cellidx(minimage(rx, P.invlx, P.lx), P.invdx, mx);
   const int ky = cellidx(minimage(ry, P.invly, P.ly), P.invdy, my);
-  double* zx = reinterpret_cast<double*>(R.z64);
-  double* zy = reinterpret_cast<double*>(R.z64 + P.nc);
+  double* zx = R.w64;
+  double* zy = R.w64 + P.nc;
   for (int ix = -w; ix <= w; ++ix) {
     const int kxn = node_wrap(kx, ix, mx);
     const double dxr = node_dist(rx, kxn, P.lx, mx, P.invlx);
@@ -172,8 +172,8 @@ __global__ void k_q2_spread(FSL_KARGS) {
         ax += -norm * dxr;
         ay += -norm * dyr;
       }
-      atomicAdd(zx + 2 * (size_t)c, ax);
-      atomicAdd(zy + 2 * (size_t)c, ay);
+      atomicAdd(zx + c, ax);
+      atomicAdd(zy + c, ay);
     }
   }
 }
@@ -185,135 +185,151 @@ __global__ void k_q2_shear(FSL_KARGS) {
   if (P.q2_shear == 0.0) return;
   const double pi2 = 2.0 * kPi;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.nc; i += gridDim.x * blockDim.x)
-    R.z64[P.nc + i].x += P.q2_shear * sin(pi2 * ((i % P.mx) / (double)P.mx));
+    R.w64[P.nc + i] += P.q2_shear * sin(pi2 * ((i % P.mx) / (double)P.mx));
 }
 
 // ------------------------------------------------------ Fourier space ---
 // Per mode: the mobility (RPY quasi-2D, src/quasi2DFunctions.cu:450-510;
 // 2-D Stokes, :767-827; Saffman-screened, :966-1035) and the stochastic
 // velocity with its Hermitian bookkeeping (:590-678, :829-904, :1037-1119).
-template <bool ONE>
-__global__ void k_q2_fourier(FSL_KARGS) {
-  FSL_REP_AT(blockIdx.y);
-  const int mx = P.mx, my = P.my, nc = P.nc, nModes = nc + mx + my;
+//
+// q2_mode: the mode at index (ix, iy) of the full spectrum, given the
+// transformed force there.
+__device__ __forceinline__ void q2_mode(const Params& P, const double* __restrict__ Rn, int ix, int iy, double2 zx, double2 zy,
+                                        double2& ox, double2& oy) {
+  const int mx = P.mx, my = P.my, nc = P.nc, nModes = nc + mx + my, i = iy * mx + ix;
   const double eta = P.eta, sigma = sqrt(P.q2_var), prefactor = P.q2_fact1;
   const bool rpy = P.scheme == 2;
   const double kc = P.q2_kc, lw = P.q2_lw;
-  const double* Rn = R.noise64;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
-    const double2 zx = R.z64[i], zy = R.z64[nc + i];
-    // deterministic: signed wave numbers with the Nyquist rows folded
-    double kx, ky;
-    {
-      int wy = i / mx, wx = i % mx;
-      if (wx > mx / 2) wx -= mx;
-      if (wy > my / 2) wy -= my;
-      const bool xh = (mx % 2) == 0 && (wx == mx / 2);
-      const bool yh = (my % 2) == 0 && (wy == my / 2);
-      if (xh && wy < 0) wx *= -1;
-      else if (yh && wx < 0) wy *= -1;
-      kx = wx * 2 * kPi / P.lx;
-      ky = wy * 2 * kPi / P.ly;
-    }
-    double oxr = 0, oxi = 0, oyr = 0, oyi = 0;
-    if (i != 0) {
-      if (rpy) {
-        const double k_inv = 1.0 / sqrt(kx * kx + ky * ky);
-        const double k3_inv = k_inv * k_inv * k_inv;
-        const double k = 1.0 / k_inv, kn = sigma * k;
-        const double f = 0.5 * (erfc(kn) * (0.5 + kn * kn) * exp(kn * kn) - kPiHalfInv * kn);
-        const double g = 0.5 * erfc(kn) * exp(kn * kn);
-        oxr = (k3_inv / eta) * (g * ky * (ky * zx.x - kx * zy.x) + f * kx * (kx * zx.x + ky * zy.x));
-        oxi = (k3_inv / eta) * (g * ky * (ky * zx.y - kx * zy.y) + f * kx * (kx * zx.y + ky * zy.y));
-        oyr = (k3_inv / eta) * (g * (-kx) * (ky * zx.x - kx * zy.x) + f * ky * (kx * zx.x + ky * zy.x));
-        oyi = (k3_inv / eta) * (g * (-kx) * (ky * zx.y - kx * zy.y) + f * ky * (kx * zx.y + ky * zy.y));
-      } else {
-        const double L = -(kx * kx) - (ky * ky);
-        double den;
-        if (kc != 0.0) {
-          const double kmod = sqrt(-L);
-          const double corr = lw != 0.0 ? tanh(kmod * lw) : 1.0;
-          den = eta * (kmod * (kmod + kc * corr));
-        } else {
-          den = -eta * L;
-        }
-        const double GWr = kx * zx.x + ky * zy.x, GWi = kx * zx.y + ky * zy.y;
-        oxr = (zx.x + kx * GWr / L) / den;
-        oxi = (zx.y + kx * GWi / L) / den;
-        oyr = (zy.x + ky * GWr / L) / den;
-        oyi = (zy.y + ky * GWi / L) / den;
-      }
-    }
-    // stochastic: canonical |wave numbers|, the noise index shared with the
-    // conjugate mode, and the flip of the conjugate's imaginary part
-    int wy = i / mx, wx = i % mx, fx = wx, fy = wy, shift = 0;
-    if (wx > mx / 2) {
-      fx = wx - mx;
-      wx = mx - wx;
-    }
-    if (wy > my / 2) {
-      fy = wy - my;
-      wy = my - wy;
-    }
-    const bool xHalf = (mx % 2) == 0 && (wx == mx / 2);
-    const bool yHalf = (my % 2) == 0 && (wy == my / 2);
-    if (xHalf && fy < 0) fx *= -1;
-    else if (yHalf && fx < 0) fy *= -1;
-    double mkx = wx * 2 * kPi / P.lx;
-    const double mky = wy * 2 * kPi / P.ly;
-    if (fx * fy < 0) {
-      shift = nModes / 2;
-      mkx *= -1.0;
-    }
-    const int index = wy * mx + wx + shift;
-    const bool edge = (xHalf && wy == 0) || (yHalf && wx == 0) || (xHalf && yHalf);
-    double Wxr = 0, Wxi = 0, Wyr = 0, Wyi = 0;
+  // deterministic: signed wave numbers with the Nyquist rows folded
+  double kx, ky;
+  {
+    int wy = iy, wx = ix;
+    if (wx > mx / 2) wx -= mx;
+    if (wy > my / 2) wy -= my;
+    const bool xh = (mx % 2) == 0 && (wx == mx / 2);
+    const bool yh = (my % 2) == 0 && (wy == my / 2);
+    if (xh && wy < 0) wx *= -1;
+    else if (yh && wx < 0) wy *= -1;
+    kx = wx * 2 * kPi / P.lx;
+    ky = wy * 2 * kPi / P.ly;
+  }
+  double oxr = 0, oxi = 0, oyr = 0, oyi = 0;
+  if (i != 0) {
     if (rpy) {
-      if (i != 0) {
-        const double k = sqrt(mkx * mkx + mky * mky);
-        const double k3half_inv = 1.0 / sqrt(k * k * k);
-        const double kn = sigma * k;
-        const double f_half = sqrt(0.5 * (erfc(kn) * (0.5 + kn * kn) * exp(kn * kn) - kPiHalfInv * kn));
-        const double g_half = sqrt(0.5 * erfc(kn) * exp(kn * kn));
-        const double a = g_half * mky, b = f_half * mkx, c = g_half * (-mkx), d = f_half * mky;
-        if (edge) {
-          Wxr = sqrt(2.0) * prefactor * k3half_inv * (a * Rn[index] + b * Rn[nModes + index]);
-          Wyr = sqrt(2.0) * prefactor * k3half_inv * (c * Rn[index] + d * Rn[nModes + index]);
-        } else {
-          Wxr = prefactor * k3half_inv * (a * Rn[index] + b * Rn[nModes + index]);
-          Wyr = prefactor * k3half_inv * (c * Rn[index] + d * Rn[nModes + index]);
-          Wxi = prefactor * k3half_inv * (a * Rn[nModes * 2 + index] + b * Rn[nModes * 3 + index]);
-          Wyi = prefactor * k3half_inv * (c * Rn[nModes * 2 + index] + d * Rn[nModes * 3 + index]);
-        }
-      }
+      const double k_inv = 1.0 / sqrt(kx * kx + ky * ky);
+      const double k3_inv = k_inv * k_inv * k_inv;
+      const double k = 1.0 / k_inv, kn = sigma * k;
+      const double f = 0.5 * (erfc(kn) * (0.5 + kn * kn) * exp(kn * kn) - kPiHalfInv * kn);
+      const double g = 0.5 * erfc(kn) * exp(kn * kn);
+      oxr = (k3_inv / eta) * (g * ky * (ky * zx.x - kx * zy.x) + f * kx * (kx * zx.x + ky * zy.x));
+      oxi = (k3_inv / eta) * (g * ky * (ky * zx.y - kx * zy.y) + f * kx * (kx * zx.y + ky * zy.y));
+      oyr = (k3_inv / eta) * (g * (-kx) * (ky * zx.x - kx * zy.x) + f * ky * (kx * zx.x + ky * zy.x));
+      oyi = (k3_inv / eta) * (g * (-kx) * (ky * zx.y - kx * zy.y) + f * ky * (kx * zx.y + ky * zy.y));
     } else {
-      const bool nyq = ((mx % 2) == 0 && (wx == mx / 2)) || ((my % 2) == 0 && (wy == my / 2)) || i == 0;
-      if (!nyq) {
-        double amp;
-        if (kc != 0.0) {
-          const double kmod2 = mkx * mkx + mky * mky, kmod = sqrt(kmod2);
-          const double corr = lw != 0.0 ? tanh(kmod * lw) : 1.0;
-          amp = 1.0 / sqrt(kmod * kmod2 * (kmod + kc * corr));
-        } else {
-          amp = 1.0 / (mkx * mkx + mky * mky);
-        }
-        if (edge) {
-          Wxr = sqrt(2.0) * prefactor * amp * (mky * Rn[index]);
-          Wyr = sqrt(2.0) * prefactor * amp * ((-mkx) * Rn[index]);
-        } else {
-          Wxr = prefactor * amp * (mky * Rn[index]);
-          Wyr = prefactor * amp * ((-mkx) * Rn[index]);
-          Wxi = prefactor * amp * (mky * Rn[nModes * 2 + index]);
-          Wyi = prefactor * amp * ((-mkx) * Rn[nModes * 2 + index]);
-        }
+      const double L = -(kx * kx) - (ky * ky);
+      double den;
+      if (kc != 0.0) {
+        const double kmod = sqrt(-L);
+        const double corr = lw != 0.0 ? tanh(kmod * lw) : 1.0;
+        den = eta * (kmod * (kmod + kc * corr));
+      } else {
+        den = -eta * L;
+      }
+      const double GWr = kx * zx.x + ky * zy.x, GWi = kx * zx.y + ky * zy.y;
+      oxr = (zx.x + kx * GWr / L) / den;
+      oxi = (zx.y + kx * GWi / L) / den;
+      oyr = (zy.x + ky * GWr / L) / den;
+      oyi = (zy.y + ky * GWi / L) / den;
+    }
+  }
+  // stochastic: canonical |wave numbers|, the noise index shared with the
+  // conjugate mode, and the flip of the conjugate's imaginary part
+  int wy = iy, wx = ix, fx = wx, fy = wy, shift = 0;
+  if (wx > mx / 2) {
+    fx = wx - mx;
+    wx = mx - wx;
+  }
+  if (wy > my / 2) {
+    fy = wy - my;
+    wy = my - wy;
+  }
+  const bool xHalf = (mx % 2) == 0 && (wx == mx / 2);
+  const bool yHalf = (my % 2) == 0 && (wy == my / 2);
+  if (xHalf && fy < 0) fx *= -1;
+  else if (yHalf && fx < 0) fy *= -1;
+  double mkx = wx * 2 * kPi / P.lx;
+  const double mky = wy * 2 * kPi / P.ly;
+  if (fx * fy < 0) {
+    shift = nModes / 2;
+    mkx *= -1.0;
+  }
+  const int index = wy * mx + wx + shift;
+  const bool edge = (xHalf && wy == 0) || (yHalf && wx == 0) || (xHalf && yHalf);
+  double Wxr = 0, Wxi = 0, Wyr = 0, Wyi = 0;
+  if (rpy) {
+    if (i != 0) {
+      const double k = sqrt(mkx * mkx + mky * mky);
+      const double k3half_inv = 1.0 / sqrt(k * k * k);
+      const double kn = sigma * k;
+      const double f_half = sqrt(0.5 * (erfc(kn) * (0.5 + kn * kn) * exp(kn * kn) - kPiHalfInv * kn));
+      const double g_half = sqrt(0.5 * erfc(kn) * exp(kn * kn));
+      const double a = g_half * mky, b = f_half * mkx, c = g_half * (-mkx), d = f_half * mky;
+      if (edge) {
+        Wxr = sqrt(2.0) * prefactor * k3half_inv * (a * Rn[index] + b * Rn[nModes + index]);
+        Wyr = sqrt(2.0) * prefactor * k3half_inv * (c * Rn[index] + d * Rn[nModes + index]);
+      } else {
+        Wxr = prefactor * k3half_inv * (a * Rn[index] + b * Rn[nModes + index]);
+        Wyr = prefactor * k3half_inv * (c * Rn[index] + d * Rn[nModes + index]);
+        Wxi = prefactor * k3half_inv * (a * Rn[nModes * 2 + index] + b * Rn[nModes * 3 + index]);
+        Wyi = prefactor * k3half_inv * (c * Rn[nModes * 2 + index] + d * Rn[nModes * 3 + index]);
       }
     }
-    if ((fx < 0) || (fx == 0 && fy < 0)) {
-      Wxi = -Wxi;
-      Wyi = -Wyi;
+  } else {
+    const bool nyq = ((mx % 2) == 0 && (wx == mx / 2)) || ((my % 2) == 0 && (wy == my / 2)) || i == 0;
+    if (!nyq) {
+      double amp;
+      if (kc != 0.0) {
+        const double kmod2 = mkx * mkx + mky * mky, kmod = sqrt(kmod2);
+        const double corr = lw != 0.0 ? tanh(kmod * lw) : 1.0;
+        amp = 1.0 / sqrt(kmod * kmod2 * (kmod + kc * corr));
+      } else {
+        amp = 1.0 / (mkx * mkx + mky * mky);
+      }
+      if (edge) {
+        Wxr = sqrt(2.0) * prefactor * amp * (mky * Rn[index]);
+        Wyr = sqrt(2.0) * prefactor * amp * ((-mkx) * Rn[index]);
+      } else {
+        Wxr = prefactor * amp * (mky * Rn[index]);
+        Wyr = prefactor * amp * ((-mkx) * Rn[index]);
+        Wxi = prefactor * amp * (mky * Rn[nModes * 2 + index]);
+        Wyi = prefactor * amp * ((-mkx) * Rn[nModes * 2 + index]);
+      }
     }
-    R.z64[i] = make_double2(oxr + Wxr, oxi + Wxi);
-    R.z64[nc + i] = make_double2(oyr + Wyr, oyi + Wyi);
+  }
+  if ((fx < 0) || (fx == 0 && fy < 0)) {
+    Wxi = -Wxi;
+    Wyi = -Wyi;
+  }
+  ox = make_double2(oxr + Wxr, oxi + Wxi);
+  oy = make_double2(oyr + Wyr, oyi + Wyi);
+}
+
+// The particles see the real part of the inverse transform, which is the
+// transform of the Hermitian part (out(k) + conj out(-k)) / 2: each thread
+// evaluates a mode of the half spectrum and its partner.
+template <bool ONE>
+__global__ void k_q2_fourier(FSL_KARGS) {
+  FSL_REP_AT(blockIdx.y);
+  const int mx = P.mx, my = P.my, mxh = P.mxh, nh = mxh * my;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
+    const int iy = i / mxh, ix = i - iy * mxh;
+    const double2 zx = R.z64[i], zy = R.z64[nh + i];
+    double2 ax, ay, bx, by;
+    q2_mode(P, R.noise64, ix, iy, zx, zy, ax, ay);
+    q2_mode(P, R.noise64, ix ? mx - ix : 0, iy ? my - iy : 0, make_double2(zx.x, -zx.y), make_double2(zy.x, -zy.y), bx, by);
+    R.z64[i] = make_double2(0.5 * (ax.x + bx.x), 0.5 * (ax.y - bx.y));
+    R.z64[nh + i] = make_double2(0.5 * (ay.x + by.x), 0.5 * (ay.y - by.y));
   }
 }
 
@@ -376,17 +392,18 @@ void launch_q2_field(const Batch& B, cudaStream_t s, Prof* prof) {
   FSL_GO(k_q2_shear, dim3(bc, B.nrep), tb, 0, s, B);
 }
 
-void launch_q2_solve(const Batch& B, cudaStream_t s, Prof* prof) {
-  const int tb = 256;
-  unsigned bc = blocks_for((long)B.nc, tb);
+void launch_q2_solve(const Batch& B, const GPlan* g, cudaStream_t s, Prof* prof) {
+  const int tb = 128;
+  unsigned bc = blocks_for((long)B.mxh * B.my, tb);
   const unsigned cap = (unsigned)((148 * 16 + B.nrep - 1) / B.nrep);
   if (bc > cap) bc = cap < 1 ? 1 : cap;
   if (prof) prof->mark(s, "q2_fft");
-  launch_fft64_2d(B, -1, s);
+  int n = launch_g_forward(B, g, 2, s);
   if (prof) prof->mark(s, "q2_fourier");
   FSL_GO(k_q2_fourier, dim3(bc, B.nrep), tb, 0, s, B);
   if (prof) prof->mark(s, "q2_fft");
-  launch_fft64_2d(B, +1, s);
+  n += launch_g_inverse(B, g, 2, 0, 1.0 / (double)B.nc, s);
+  if (prof) prof->count(n + 1);
 }
 
 void launch_q2_update(const Batch& B, int stage, cudaStream_t s) {
