@@ -283,41 +283,6 @@ __device__ __forceinline__ int stencil_base(const Params& P, int d, int face, do
   return cellidx(minimage(r, invL, L), invd, m);
 }
 
-// Warp-shared stencil of one particle for all three components.  Per
-// dimension d there are two node families: cell centres (components with
-// comp != d) and faces (comp == d); with n nodes each that is 6n values,
-// lane (f * 3 + d) * n + k computing family f, dimension d, node k.  Every
-// lane calls this; the result stays in the computing lane and is read with
-// stencil_get.
-struct WarpStencil {
-  int j;
-  float w;
-};
-
-__device__ __forceinline__ WarpStencil warp_stencil(const Params& P, const double posc[3],
-                                                    const double posw[3], int lane) {
-  WarpStencil s{0, 0.0f};
-  const int n = P.kernel;
-  if (lane < 6 * n) {
-    int k = lane % n, fd = lane / n;
-    int f = fd / 3, d = fd - 3 * f;
-    // selects, not posc[d]: a runtime index would put the arrays on the stack
-    const double pc = d == 0 ? posc[0] : (d == 1 ? posc[1] : posc[2]);
-    const double pw = d == 0 ? posw[0] : (d == 1 ? posw[1] : posw[2]);
-    // family f = 1 is the face family of dimension d: use comp = d
-    stencil_node(P, d, f == 1 ? d : (d + 1) % 3, pc, pw, k, s.j, s.w);
-  }
-  return s;
-}
-
-// node k of dimension d for component comp, from the lanes of warp_stencil
-__device__ __forceinline__ void stencil_get(const WarpStencil& s, int n, int comp, int d, int k,
-                                            int& j, float& w) {
-  int src = ((comp == d ? 3 : 0) + d) * n + k;
-  j = __shfl_sync(0xffffffffu, s.j, src);
-  w = __shfl_sync(0xffffffffu, s.w, src);
-}
-
 __device__ __forceinline__ void set_err(int* err, int bit) {
   atomicOr(&err[ERR_BITS], bit);
   err[ERR_ANY] = 1;

@@ -1116,6 +1116,22 @@ __device__ __forceinline__ void quad_spread(const Params& P, const QuadStencil<K
   }
 }
 
+// The sum of w v over the z nodes of one (x, y) node pair: even and odd
+// nodes apart, then their sum.  Quads and whole warps (interp_wide) add the
+// nodes of a particle in this one order: z (even, odd), y (0+1, 2+3), x
+// (0+1, 2+3), so both give the same bits.
+__device__ __forceinline__ float interp_term(float wx, float wy, float wz, float v) { return __fmul_rn(wx * (wy * wz), v); }
+__device__ __forceinline__ float interp_term(float wx, float wy, float wz, float v, float s) {
+  return __fmaf_rn(wx * (wy * wz), v, s);
+}
+template <int KN>
+__device__ __forceinline__ float interp_row(float wx, float wy, const float (&wz)[KN], const float* v) {
+  const float e = interp_term(wx, wy, wz[2], v[2], interp_term(wx, wy, wz[0], v[0]));
+  float o = interp_term(wx, wy, wz[1], v[1]);
+  if (KN == 4) o = interp_term(wx, wy, wz[KN - 1], v[KN - 1], o);
+  return e + o;
+}
+
 // J v of one particle by its quad: each lane sums w v over its nodes per
 // component, then the quad adds its four partial sums (xor 1, then xor 2);
 // every lane of the quad gets the three sums
@@ -1134,11 +1150,11 @@ __device__ __forceinline__ void quad_interp(const Params& P, const QuadStencil<K
 #pragma unroll
       for (int c = 0; c < KN; ++c)
         val[b * KN + c] = a < KN ? __ldg(vc + (x + P.mx * (S.jy[comp == 1][b] + P.my * S.jz[comp == 2][c]))) : 0.0f;
-    float s = 0.0f;
+    float row[KN];
 #pragma unroll
     for (int b = 0; b < KN; ++b)
-#pragma unroll
-      for (int c = 0; c < KN; ++c) s += (wx * (S.wy[comp == 1][b] * S.wz[comp == 2][c])) * val[b * KN + c];
+      row[b] = interp_row<KN>(wx, S.wy[comp == 1][b], S.wz[comp == 2], val + b * KN);
+    float s = KN == 4 ? (row[0] + row[1]) + (row[2] + row[KN - 1]) : (row[0] + row[1]) + row[2];
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
     u[comp] = s;
@@ -1406,6 +1422,183 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_spread(FSL_KARGS, int drift
   if (sat) set_err(R.err, 1);
 }
 
+// ------------------------------------------------- one warp per particle ---
+// The spread and the interpolation of launches with few particles.  A quad
+// runs its particle's stencil as one chain (six FP64 nodes, then 16 or 48
+// products a lane, and the spread's box to clear and flush), and with a few
+// hundred particles the GPU holds a few dozen warps, so the launch takes that
+// chain's latency.  Here a warp takes one particle: lane (f 3 + d) KN + k
+// computes node k of family f in dimension d, the nodes go round by shuffles,
+// and lane a + 4 b + 16 c0 handles the x node a, the y node b and the z nodes
+// c0, c0 + 2 of every component.  Forces are quad_force_vl's, taken by all
+// eight quads of the warp alike.  Same products, same integer sums, same
+// order of every FP32 and FP64 sum: the bits of the quad kernels.
+// Launches of at most this many quad blocks (64 particles each) take it: one
+// block per SM.  A step of 64^3 cells, 4-point kernel: 512 particles 127 us
+// with quads, 98 us with warps; 4,096: 132 and 108; 8,192: 133 and 121;
+// 16,384: 140 and 147; 32,768: 159 and 204.
+constexpr unsigned kWideBlocks = 148;
+
+struct WideLane {
+  int j;
+  float w;
+};
+
+template <int KN>
+__device__ __forceinline__ WideLane wide_lane(const Params& P, const double posc[3], const double posw[3], int lane) {
+  WideLane s{0, 0.0f};
+  if (lane < 6 * KN) {
+    const int k = lane % KN, fd = lane / KN, f = fd / 3, d = fd - 3 * f;
+    // selects, not posc[d]: a runtime index would put the arrays on the stack
+    const double pc = d == 0 ? posc[0] : (d == 1 ? posc[1] : posc[2]);
+    const double pw = d == 0 ? posw[0] : (d == 1 ? posw[1] : posw[2]);
+    stencil_node(P, d, f == 1 ? d : (d + 1) % 3, pc, pw, k, s.j, s.w);
+  }
+  return s;
+}
+
+// The nodes of one lane: x node a, y node b, z nodes c0 and c0 + 2 of both
+// families (0: cell centres, 1: faces).
+struct WideNodes {
+  int jx[2], jy[2], jz[2][2];
+  float wx[2], wy[2], wz[2][2];
+  bool on[2];  // whether the products with z node c0, c0 + 2 exist
+};
+
+template <int KN>
+__device__ __forceinline__ void wide_share(const WideLane& s, int lane, WideNodes& N) {
+  const int a = lane & 3, b = (lane >> 2) & 3, c0 = lane >> 4;
+  const int ka = min(a, KN - 1), kb = min(b, KN - 1), kc = min(c0 + 2, KN - 1);
+#pragma unroll
+  for (int f = 0; f < 2; ++f) {
+    const int at = 3 * f * KN;
+    N.jx[f] = __shfl_sync(0xffffffffu, s.j, at + ka);
+    N.wx[f] = __shfl_sync(0xffffffffu, s.w, at + ka);
+    N.jy[f] = __shfl_sync(0xffffffffu, s.j, at + KN + kb);
+    N.wy[f] = __shfl_sync(0xffffffffu, s.w, at + KN + kb);
+    N.jz[f][0] = __shfl_sync(0xffffffffu, s.j, at + 2 * KN + c0);
+    N.wz[f][0] = __shfl_sync(0xffffffffu, s.w, at + 2 * KN + c0);
+    N.jz[f][1] = __shfl_sync(0xffffffffu, s.j, at + 2 * KN + kc);
+    N.wz[f][1] = __shfl_sync(0xffffffffu, s.w, at + 2 * KN + kc);
+  }
+  N.on[0] = a < KN && b < KN;
+  N.on[1] = N.on[0] && c0 + 2 < KN;
+}
+
+// The products of one particle (quad_spread's, spread over the warp).
+__device__ __forceinline__ void wide_spread(const Params& P, const WideNodes& N, const double val[3],
+                                            unsigned long long* __restrict__ grid, bool& sat) {
+  const bool fatom = P.prec == PREC_FLOAT;
+#pragma unroll
+  for (int comp = 0; comp < 3; ++comp) {
+    const double vc = val[comp];
+    if (vc == 0.0) continue;
+    const double vs = vc * kFixedScale;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (!N.on[c]) continue;
+      const int at = N.jx[comp == 0] + P.mx * (N.jy[comp == 1] + P.my * N.jz[comp == 2][c]);
+      const float w = N.wx[comp == 0] * (N.wy[comp == 1] * N.wz[comp == 2][c]);
+      if (fatom) {
+        const float fv = (float)((double)w * vc);
+        if (fv != 0.0f) atomicAdd(reinterpret_cast<float*>(grid) + (size_t)comp * P.nc + at, fv);
+        continue;
+      }
+      const double v = (double)w * vs;
+      sat |= !(fabs(v) < kFixedMax);
+      const long long iv = sat ? 0ll : __double2ll_rn(v);
+      if (iv != 0) atomicAdd(grid + (size_t)comp * P.nc + at, (unsigned long long)iv);
+    }
+  }
+}
+
+template <bool ONE, int KN>
+__global__ void __launch_bounds__(kPartThreads) k_spread_wide(FSL_KARGS, int drift, int ordered, int forces, int cache) {
+  FSL_REP_FLAT(KIND_T32);
+  const int np = P.np;
+  const bool own_forces = forces && (P.verlet || P.nolist);
+  const bool cell_mode = own_forces ? vl_state(R, blk) : false;
+  const int lane = threadIdx.x & 31;
+  const long e = (blk * (long)blockDim.x + threadIdx.x) >> 5;
+  if (e >= np) return;  // a whole warp
+  const bool by_cell = ordered && !P.verlet && !P.nolist;
+  const int i = by_cell ? cell_list(R, drift == 1).sorted[e] : (int)e;
+  bool sat = false;
+  {
+    const double* qf = drift == 1 ? R.qp : R.q;
+    const double pos[3] = {qf[i], qf[np + i], qf[2 * np + i]};
+    double val[3];
+    if (own_forces) {
+      quad_force_vl(P, R, i, lane & 3, drift == 1 ? 1 : 0, true, cell_mode, val[0], val[1], val[2]);
+      if (lane == 0) {
+        if (!isfinite(val[0]) || !isfinite(val[1]) || !isfinite(val[2])) set_err(R.err, 2);
+        R.F[i] = val[0];
+        R.F[np + i] = val[1];
+        R.F[2 * (size_t)np + i] = val[2];
+      }
+    } else {
+      val[0] = R.F[i];
+      val[1] = R.F[np + i];
+      val[2] = R.F[2 * (size_t)np + i];
+    }
+    const WideLane L = wide_lane<KN>(P, pos, pos, lane);
+    if (cache && R.stc && lane < 6 * KN) {
+      // words fd (node) and 6 + fd (weight) of lane slot 4 i + k (lane_store)
+      const int k = lane % KN, fd = lane / KN;
+      const size_t np4 = (size_t)4 * np, slot = (size_t)4 * i + k;
+      unsigned* st = reinterpret_cast<unsigned*>(R.stc);
+      st[((fd >> 2) * np4 + slot) * 4 + (fd & 3)] = (unsigned)L.j;
+      st[(((6 + fd) >> 2) * np4 + slot) * 4 + ((6 + fd) & 3)] = __float_as_uint(L.w);
+    }
+    WideNodes N;
+    wide_share<KN>(L, lane, N);
+    wide_spread(P, N, val, R.grid, sat);
+  }
+  if (drift) {
+    double W[3], pos[3], pp[3], pm[3], vp[3], vm[3];
+    rfd_inputs(P, R, i, W, pos);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      pp[d] = pos[d] + 0.5 * kRfdDelta * W[d];
+      pm[d] = pos[d] - 0.5 * kRfdDelta * W[d];
+      vp[d] = (P.kT / kRfdDelta) * W[d];
+      vm[d] = (P.kT / kRfdDelta) * -1 * W[d];
+    }
+    bool any = true;
+    if (P.rfd != 1) {
+      // reference mode: only components whose displaced nodes differ
+      // (rfd_drift_at)
+      bool diff = false;
+      if (lane < 6) {
+        const int f = lane / 3, d = lane - 3 * f;
+        const double x = d == 0 ? pp[0] : (d == 1 ? pp[1] : pp[2]);
+        const double y = d == 0 ? pm[0] : (d == 1 ? pm[1] : pm[2]);
+        diff = stencil_base(P, d, f, x) != stencil_base(P, d, f, y);
+      }
+      const unsigned chg = __ballot_sync(0xffffffffu, diff);
+      any = chg != 0;
+      constexpr unsigned fam[3] = {(1 << 3) | (1 << 1) | (1 << 2), (1 << 4) | (1 << 0) | (1 << 2),
+                                   (1 << 5) | (1 << 0) | (1 << 1)};
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        if (!(chg & fam[c])) vp[c] = vm[c] = 0.0;
+    }
+    if (any) {  // warp-uniform
+      WideNodes N;
+      wide_share<KN>(wide_lane<KN>(P, pp, P.rfd == 1 ? pp : pos, lane), lane, N);
+      wide_spread(P, N, vp, R.grid, sat);
+      wide_share<KN>(wide_lane<KN>(P, pm, P.rfd == 1 ? pm : pos, lane), lane, N);
+      wide_spread(P, N, vm, R.grid, sat);
+    }
+  }
+  if (sat) set_err(R.err, 1);
+}
+
+// Whether a launch takes one warp per particle.
+static bool wide_particles(const Batch& B) {
+  return part_blocks(B, KIND_T4) <= kWideBlocks;
+}
+
 // FLUAMSL_SPREAD_BOX=0 spreads every product with its own global atomic (the
 // same sums, for comparison)
 static int spread_box() {
@@ -1419,8 +1612,16 @@ static int spread_box() {
 void launch_spread(const Batch& B, int drift, int ordered, cudaStream_t s, bool forces, bool cache) {
   if (B.max_np == 0) return;
   if (B.prec == PREC_F64) return launch_spread64(B, drift, s);
-  const unsigned g = part_blocks(B, KIND_T4);
   const int f = forces ? 1 : 0, c = cache ? 1 : 0;
+  if (wide_particles(B)) {
+    const unsigned w = part_blocks(B, KIND_T32);
+    if (B.kernel == 4)
+      FSL_GO_T(k_spread_wide, 4, w, kPartThreads, 0, s, B, drift, ordered, f, c);
+    else
+      FSL_GO_T(k_spread_wide, 3, w, kPartThreads, 0, s, B, drift, ordered, f, c);
+    return;
+  }
+  const unsigned g = part_blocks(B, KIND_T4);
   if (B.kernel == 4)
     FSL_GO_T(k_spread, 4, g, kPartThreads, 0, s, B, drift, ordered, spread_box(), f, c);
   else
@@ -1812,6 +2013,77 @@ __global__ void k_interp_update(FSL_KARGS, int stage, int cached) {
   qout[k] = r;
 }
 
+// The same by one warp per particle (k_spread_wide's layout and rule).
+template <bool ONE, int KN>
+__global__ void __launch_bounds__(kPartThreads) k_interp_wide(FSL_KARGS, int stage, int cached) {
+  FSL_REP_FLAT(KIND_T32);
+  const int np = P.np, lane = threadIdx.x & 31;
+  const long e = (blk * (long)blockDim.x + threadIdx.x) >> 5;
+  if (e >= np) return;  // a whole warp
+  const int i = (int)e;
+  const double* qpos = stage == 1 ? R.q : R.qp;
+  double* qout = stage == 1 ? R.qp : R.q;
+  WideLane L{0, 0.0f};
+  if (cached && R.stc) {
+    if (lane < 6 * KN) {
+      const int k = lane % KN, fd = lane / KN;
+      const size_t np4 = (size_t)4 * np, slot = (size_t)4 * i + k;
+      const unsigned* st = reinterpret_cast<const unsigned*>(R.stc);
+      L.j = (int)__ldg(st + ((fd >> 2) * np4 + slot) * 4 + (fd & 3));
+      L.w = __uint_as_float(__ldg(st + (((6 + fd) >> 2) * np4 + slot) * 4 + ((6 + fd) & 3)));
+    }
+  } else {
+    const double pos[3] = {qpos[i], qpos[np + i], qpos[2 * np + i]};
+    L = wide_lane<KN>(P, pos, pos, lane);
+  }
+  // what the update needs, on its way while the nodes go round
+  const int comp = (lane & 3) < 3 ? lane & 3 : 0;
+  const size_t k = (size_t)comp * np + i;
+  const double q0 = R.q[k];
+  WideNodes N;
+  wide_share<KN>(L, lane, N);
+  float val[3][2];
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      val[d][c] = N.on[c] ? __ldg(R.v + (size_t)d * P.nc + (N.jx[d == 0] + P.mx * (N.jy[d == 1] + P.my * N.jz[d == 2][c]))) : 0.0f;
+  float us[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    // interp_row's and quad_interp's order: z, y, x
+    float s = interp_term(N.wx[d == 0], N.wy[d == 1], N.wz[d == 2][0], val[d][0]);
+    if (N.on[1]) s = interp_term(N.wx[d == 0], N.wy[d == 1], N.wz[d == 2][1], val[d][1], s);
+    if (!N.on[0]) s = 0.0f;
+    s += __shfl_xor_sync(0xffffffffu, s, 16);
+    s += __shfl_xor_sync(0xffffffffu, s, 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 8);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    us[d] = s;
+  }
+  const double u = (double)(comp == 0 ? us[0] : (comp == 1 ? us[1] : us[2]));
+  const double h = stage == 1 ? 0.5 * P.dt : P.dt;
+  double r = q0 + h * u;
+  if (P.has_extra) {
+    const size_t nb = (size_t)6 * P.nc + (size_t)(3 + comp) * np + i;
+    double xi = (double)R.noise[nb];
+    if (stage == 2) xi += (double)R.noise[nb + (size_t)3 * np];
+    r += h * P.extra_mob * R.F[k] + P.fact2 * xi;
+  }
+  if (P.verlet) {
+    // k_interp_update's rebuild test
+    const double d = (lane & 3) < 3 ? r - R.qref[k] : 0.0;
+    double d2 = d * d;
+    d2 += __shfl_xor_sync(0xffffffffu, d2, 1);
+    d2 += __shfl_xor_sync(0xffffffffu, d2, 2);
+    if (lane == 0 && d2 > P.vl_half2) R.vl_flag[stage == 1 ? 1 : 0] = *R.t + stage;
+  }
+  if (lane >= 3) return;
+  if (!isfinite(r)) set_err(R.err, 2);
+  qout[k] = r;
+}
+
 template <bool ONE, int KN>
 __global__ void k_interp(FSL_KARGS) {
   FSL_REP_FLAT(KIND_T4);
@@ -1832,8 +2104,16 @@ __global__ void k_interp(FSL_KARGS) {
 void launch_interp_update(const Batch& B, int stage, cudaStream_t s, bool cached) {
   if (B.max_np == 0) return;
   if (B.prec == PREC_F64) return launch_interp_update64(B, stage, s);
-  const unsigned g = part_blocks(B, KIND_T4);
   const int c = cached ? 1 : 0;
+  if (wide_particles(B)) {
+    const unsigned w = part_blocks(B, KIND_T32);
+    if (B.kernel == 4)
+      FSL_GO_T(k_interp_wide, 4, w, kPartThreads, 0, s, B, stage, c);
+    else
+      FSL_GO_T(k_interp_wide, 3, w, kPartThreads, 0, s, B, stage, c);
+    return;
+  }
+  const unsigned g = part_blocks(B, KIND_T4);
   if (B.kernel == 4)
     FSL_GO_T(k_interp_update, 4, g, kPartThreads, 0, s, B, stage, c);
   else
