@@ -89,9 +89,11 @@ SlotLayout layout(const Params& P, int np_cap) {
   L.start1 = take(two_lists ? sizeof(int) * (mN + 1) : 0);
   L.sorted1 = take(two_lists ? sizeof(int) * np : 0);
   L.ws1 = take(two_lists ? sizeof(double) * 3 * np : 0);
-  L.vl_cnt = take(P.verlet ? sizeof(int) * np : 0);
-  L.vl_idx = take(P.verlet ? sizeof(int) * (size_t)kVlCap * np : 0);
-  L.qref = take(P.verlet ? sizeof(double) * 3 * np : 0);
+  // for every pair potential: a slot of a server's class may serve a request
+  // without a Verlet list first and one with it later
+  L.vl_cnt = take(two_lists ? sizeof(int) * np : 0);
+  L.vl_idx = take(two_lists ? sizeof(int) * (size_t)kVlCap * np : 0);
+  L.qref = take(two_lists ? sizeof(double) * 3 * np : 0);
   L.vl_flag = take(sizeof(uint64_t) * 3);
   L.bar = take(sizeof(unsigned) * 2);
   L.total = off;
@@ -373,9 +375,9 @@ int slot_alloc(Slot& s, const Params& P, int np_cap, cudaStream_t st) {
   r.start1 = two_lists ? (int*)(base + L.start1) : nullptr;
   r.sorted1 = two_lists ? (int*)(base + L.sorted1) : nullptr;
   r.ws1 = two_lists ? (double*)(base + L.ws1) : nullptr;
-  r.vl_cnt = P.verlet ? (int*)(base + L.vl_cnt) : nullptr;
-  r.vl_idx = P.verlet ? (int*)(base + L.vl_idx) : nullptr;
-  r.qref = P.verlet ? (double*)(base + L.qref) : nullptr;
+  r.vl_cnt = two_lists ? (int*)(base + L.vl_cnt) : nullptr;
+  r.vl_idx = two_lists ? (int*)(base + L.vl_idx) : nullptr;
+  r.qref = two_lists ? (double*)(base + L.qref) : nullptr;
   r.vl_flag = (uint64_t*)(base + L.vl_flag);
   r.bar = (unsigned*)(base + L.bar);  // zeroed with the slot
   return FSL_OK;
@@ -1106,6 +1108,8 @@ int exec_prepare(Exec& e) {
     shape.push_back(g.prof.on ? 1 : 0);
     shape.push_back((long long)(uintptr_t)g.io_in);
     shape.push_back((long long)(uintptr_t)g.io_out);
+    // the pair path of the instances and the list build launch other kernels
+    shape.push_back(g.B.has_vl | g.B.has_cl << 1 | (g.B.lists_pick + 1) << 2);
     for (int k = 0; k < NKIND; ++k) shape.push_back(g.B.nblk[k]);
     // a single instance is a by-value kernel argument: any change to it
     // needs a new capture
