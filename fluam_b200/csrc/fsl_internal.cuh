@@ -54,7 +54,7 @@ struct Params {
   int scheme;  // FSL_SCHEME_* (0 midpoint, 1 first order, 2 quasi2D, 3 stokesLimit2D)
   int prec;    // FSL_PRECISION_* (0 fixed point, 1 float atomics, 2 FP64)
   int observe; // FP64 observables accumulated at the end of every step
-  // pair forces from a Verlet list (soft repulsion): pairs within
+  // pair forces from a Verlet list: pairs within
   // rc + skin at the reference positions qref, rebuilt when a particle has
   // moved more than skin / 2 since; nolist: no pair forces, no cell list
   int verlet, nolist;

@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_forces(FSL_KARGS, int which
 }
 
 // ------------------------------------------------------------ Verlet list ---
-// Soft repulsion has an explicit cutoff, so its pair forces can come from a
+// Both pair forces are zero from the cutoff on, so they can come from a
 // list of the pairs within rc + skin at reference positions qref: every pair
 // within rc at positions that moved at most skin / 2 from qref is on it.
 // The list is rebuilt from a cell list of the current positions (the cells
@@ -814,10 +814,14 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
       bond_force(rx, ry, rz, p[0], p[1], p[2], R.bfp_k[off + j], R.bfp_r0[off + j], fx, fy, fz);
     }
   }
+  const double c1 = 2.0 * P.soft_eps / P.cutoff, c2 = 1.0 / P.cutoff;
+  // the force over r of a pair within the cutoff
+  auto pair = [&](double r2) {
+    return P.pair == 1 ? (double)tex_linear(R.ljtab, kLjTableSize, (float)(r2 * P.invcut2)) : c1 * (rsqrt(r2) - c2);
+  };
   if (P.verlet && on && cell_mode) {
     // the 27 neighbour cells of the current cell list, lanes taking cells
     // a, a + 4, ...
-    const double c1 = 2.0 * P.soft_eps / P.cutoff, c2 = 1.0 / P.cutoff;
     const CellList cl = cell_list(R, which);
     const int cx = cellidx(minimage(rx, P.invlx, P.lx), P.invdnx, P.mnx),
               cy = cellidx(minimage(ry, P.invly, P.ly), P.invdny, P.mny),
@@ -833,14 +837,13 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
         const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rxij, rxij), __dmul_rn(ryij, ryij)),
                                     __dmul_rn(rzij, rzij));
         if (j == i || r2 >= P.cutoff2 || r2 == 0.0) continue;
-        const double f = c1 * (rsqrt(r2) - c2);
+        const double f = pair(r2);
         fx += f * rxij;
         fy += f * ryij;
         fz += f * rzij;
       }
     }
   } else if (P.verlet && on) {
-    const double c1 = 2.0 * P.soft_eps / P.cutoff, c2 = 1.0 / P.cutoff;
     const int n = R.vl_cnt[i];
     for (int k = a; k < n; k += 4) {
       const int j = R.vl_idx[(size_t)k * np + i];
@@ -850,7 +853,7 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
       const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rxij, rxij), __dmul_rn(ryij, ryij)),
                                   __dmul_rn(rzij, rzij));
       if (r2 >= P.cutoff2 || r2 == 0.0) continue;
-      const double f = c1 * (rsqrt(r2) - c2);
+      const double f = pair(r2);
       fx += f * rxij;
       fy += f * ryij;
       fz += f * rzij;
@@ -874,7 +877,7 @@ __device__ __forceinline__ bool vl_state(const Rep& R, int blk) {
   return cell_mode;
 }
 
-// Pair forces from the Verlet list (soft repulsion with the cutoff test and
+// Pair forces from the Verlet list (with the cutoff test and
 // arithmetic of k_forces, on the minimum image of the unwrapped positions as
 // the reference takes it) plus the bonded forces; one quad per particle
 // (quad_force_vl).  Also the force kernel of instances without pair forces
