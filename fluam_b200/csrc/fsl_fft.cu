@@ -502,10 +502,11 @@ FftPlan* fft_plan_create(const Params& P) {
     else fp->zsolve_r[0] = fp->zsolve_r[1] = nullptr;
   }
   // the five-pass schedule needs the register plane shapes (the same
-  // packing) and the register z pass; it starts as the default where it
-  // exists, and fft_autotune keeps whichever is faster
+  // packing) and the register z pass; fft_autotune takes it where it is
+  // faster, the plane schedule serves until then (and classes that are never
+  // tuned: a server's later ones, whose first step is captured)
   if (!fp->plane_fwd_r[0] || !fp->zsolve_r[0]) fp->line_xf[0] = fp->line_xf[1] = nullptr;
-  fp->use_lines = fp->line_xf[0] != nullptr && sched_env() != 1;
+  fp->use_lines = fp->line_xf[0] != nullptr && sched_env() == 2;
   cudaGetLastError();
   if (fp->plane_fwd_r[0] || fp->zsolve_r[0]) {
     // small-DFT coefficient tables (idempotent)

@@ -469,10 +469,12 @@ int slot_reset(Slot& s, const Params& P, const double* q, const fsl_config& c, c
     FSL_TRY(cudaMemcpyAsync(r.q, q, sizeof(double) * n3p, cudaMemcpyHostToDevice, st));
     FSL_TRY(cudaMemcpyAsync(r.qp, q, sizeof(double) * n3p, cudaMemcpyHostToDevice, st));
   }
-  std::vector<float> tab;
-  build_ljtable(P, c.temperature, c.cutoff, tab);
-  // pageable source: the copy is staged before the call returns
-  FSL_TRY(cudaMemcpyAsync(r.ljtab, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice, st));
+  if (P.pair == FSL_PAIR_TABLE_LJ) {
+    std::vector<float> tab;
+    build_ljtable(P, c.temperature, c.cutoff, tab);
+    // pageable source: the copy is staged before the call returns
+    FSL_TRY(cudaMemcpyAsync(r.ljtab, tab.data(), sizeof(float) * tab.size(), cudaMemcpyHostToDevice, st));
+  }
   FSL_TRY(cudaMemsetAsync(r.F, 0, sizeof(double) * 3 * cap, st));
   FSL_TRY(cudaMemsetAsync(r.bpp_cnt, 0, sizeof(int) * cap, st));
   FSL_TRY(cudaMemsetAsync(r.bpp_off, 0, sizeof(int) * cap, st));
@@ -608,7 +610,15 @@ int group_init(Group& g, const Params& P0) {
   return FSL_OK;
 }
 
+static void group_drop_graph(Group& g) {
+  if (g.gexec) cudaGraphExecDestroy(g.gexec);
+  if (g.graph) cudaGraphDestroy(g.graph);
+  g.gexec = nullptr;
+  g.graph = nullptr;
+}
+
 void group_destroy(Group& g) {
+  group_drop_graph(g);
   if (g.side) {
     cudaStreamSynchronize(g.side);
     cudaStreamDestroy(g.side);
@@ -1082,7 +1092,8 @@ void exec_destroy(Exec& e) {
 
 namespace {
 
-int exec_prepare(Exec& e) {
+// A stream per group and an event per stream.
+int exec_streams(Exec& e) {
   const size_t ng = e.groups.size();
   while (e.side.size() + 1 < ng) {
     cudaStream_t s;
@@ -1096,6 +1107,33 @@ int exec_prepare(Exec& e) {
     FSL_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     e.ev.push_back(ev);
   }
+  return FSL_OK;
+}
+
+// What a captured step of g depends on.
+void group_shape(const Group& g, std::vector<long long>& shape) {
+  shape.push_back((long long)(uintptr_t)g.B.reps);
+  shape.push_back(g.B.nrep);
+  shape.push_back(g.B.max_np);
+  shape.push_back((long long)g.B.max_noise_n);
+  shape.push_back(g.prof.on ? 1 : 0);
+  shape.push_back((long long)(uintptr_t)g.io_in);
+  shape.push_back((long long)(uintptr_t)g.io_out);
+  // the pair path of the instances and the list build launch other kernels
+  shape.push_back(g.B.has_vl | g.B.has_cl << 1 | (g.B.lists_pick + 1) << 2);
+  for (int k = 0; k < NKIND; ++k) shape.push_back(g.B.nblk[k]);
+  // a single instance is a by-value kernel argument: any change to it
+  // needs a new capture
+  if (g.B.one) {
+    long long w[(sizeof(Rep) + 7) / 8] = {};
+    std::memcpy(w, g.B.one, sizeof(Rep));
+    shape.insert(shape.end(), w, w + (sizeof(Rep) + 7) / 8);
+  }
+}
+
+int exec_prepare(Exec& e) {
+  const size_t ng = e.groups.size();
+  if (int rc = exec_streams(e)) return rc;
   std::vector<long long> shape;
   shape.push_back((long long)(uintptr_t)e.io_key[0]);
   shape.push_back((long long)(uintptr_t)e.io_key[1]);
@@ -1109,23 +1147,7 @@ int exec_prepare(Exec& e) {
     g.stream = i == 0 ? e.stream : e.side[i - 1];
     int rc = group_upload(g);
     if (rc) return rc;
-    shape.push_back((long long)(uintptr_t)g.B.reps);
-    shape.push_back(g.B.nrep);
-    shape.push_back(g.B.max_np);
-    shape.push_back((long long)g.B.max_noise_n);
-    shape.push_back(g.prof.on ? 1 : 0);
-    shape.push_back((long long)(uintptr_t)g.io_in);
-    shape.push_back((long long)(uintptr_t)g.io_out);
-    // the pair path of the instances and the list build launch other kernels
-    shape.push_back(g.B.has_vl | g.B.has_cl << 1 | (g.B.lists_pick + 1) << 2);
-    for (int k = 0; k < NKIND; ++k) shape.push_back(g.B.nblk[k]);
-    // a single instance is a by-value kernel argument: any change to it
-    // needs a new capture
-    if (g.B.one) {
-      long long w[(sizeof(Rep) + 7) / 8] = {};
-      std::memcpy(w, g.B.one, sizeof(Rep));
-      shape.insert(shape.end(), w, w + (sizeof(Rep) + 7) / 8);
-    }
+    group_shape(g, shape);
   }
   if (shape != e.shape) {
     exec_drop_graph(e);
@@ -1224,6 +1246,51 @@ int exec_step(Exec& e, int64_t nsteps) {
       if (rc) return rc;
     }
   }
+  return FSL_OK;
+}
+
+int exec_step_each(Exec& e, int64_t nsteps) {
+  if (nsteps < 0) return errorf(FSL_E_ARG, "negative step count");
+  FSL_TRY(cudaSetDevice(e.device));
+  if (nsteps == 0 || e.groups.empty()) return FSL_OK;
+  // the first step of an Exec runs eagerly and tunes its classes
+  if (e.steps == 0) {
+    if (int rc = exec_step(e, 1)) return rc;
+    if (--nsteps == 0) return FSL_OK;
+  }
+  const size_t ng = e.groups.size();
+  if (int rc = exec_streams(e)) return rc;
+  // the groups' streams take up after what is queued on the main one (new
+  // instances' buffers)
+  FSL_TRY(cudaEventRecord(e.ev[0], e.stream));
+  int total = 0;
+  for (size_t i = 0; i < ng; ++i) {
+    Group& g = *e.groups[i];
+    g.stream = i == 0 ? e.stream : e.side[i - 1];
+    if (i > 0) FSL_TRY(cudaStreamWaitEvent(g.stream, e.ev[0], 0));
+    if (int rc = group_upload(g)) return rc;
+    std::vector<long long> shape;
+    group_shape(g, shape);
+    if (!g.gexec || shape != g.shape) {
+      group_drop_graph(g);
+      g.shape = shape;
+      FSL_TRY(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
+      group_enqueue_step(g);
+      const cudaError_t ce = cudaStreamEndCapture(g.stream, &g.graph);
+      if (ce != cudaSuccess) return cuda_fail(ce, "graph capture");
+      FSL_TRY(cudaGraphInstantiate(&g.gexec, g.graph, 0));
+      e.captures++;
+    }
+    total += g.launches;
+  }
+  e.launches_per_step = total;
+  for (int64_t k = 0; k < nsteps; ++k)
+    for (Group* g : e.groups) FSL_TRY(cudaGraphLaunch(g->gexec, g->stream));
+  for (size_t i = 1; i < ng; ++i) {
+    FSL_TRY(cudaEventRecord(e.ev[i], e.side[i - 1]));
+    FSL_TRY(cudaStreamWaitEvent(e.stream, e.ev[i], 0));
+  }
+  e.steps += (uint64_t)nsteps;
   return FSL_OK;
 }
 

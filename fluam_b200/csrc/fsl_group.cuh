@@ -126,6 +126,11 @@ struct Group {
   // after forking its noise
   cudaEvent_t io_wait = nullptr;
   const char* fail_stage = nullptr;  // first stage whose launch failed
+  // the group's own captured step and what it was captured for
+  // (exec_step_each)
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t gexec = nullptr;
+  std::vector<long long> shape;
 };
 
 int group_init(Group& g, const Params& P0);
@@ -172,6 +177,12 @@ void exec_drop_graph(Exec& e);
 // nsteps midpoint steps of every group; the first step of an Exec runs
 // eagerly, later ones replay the captured graph.
 int exec_step(Exec& e, int64_t nsteps);
+
+// The same with a graph per group, each on the group's stream: the groups run
+// their steps side by side without waiting for one another before the last,
+// and a set of groups that changes between calls captures nothing anew (the
+// server: classes come and go with their requests).
+int exec_step_each(Exec& e, int64_t nsteps);
 
 // src/initForcesNonBonded.cu:21-53 (float accumulation, float sqrt,
 // sigma = 2 dx, epsilon = kT, first and last entries zero).

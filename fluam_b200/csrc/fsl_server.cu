@@ -2,9 +2,11 @@
 // that admits queued requests into slots of their size class under a device
 // memory budget and steps every admitted request together (continuous
 // batching).  The slot of a finished request is switched off in its group's
-// instance table and handed to the next request of the class, so the
-// captured step graph stays valid; only a group whose slot list grows or
-// shrinks needs a new capture.
+// instance table and handed to the next request of the class, so the class's
+// captured step graph stays valid; only a class whose slot list grows or
+// shrinks needs a new capture (exec_step_each: one graph per class; with one
+// graph over all classes every class that came or went cost a capture of
+// them all).
 #include <algorithm>
 #include <array>
 #include <chrono>
@@ -45,13 +47,8 @@ struct SGroup {
   std::vector<std::unique_ptr<fsl::Slot>> slots;
   std::vector<Request*> owner;  // per slot; nullptr = free
   int busy = 0;
-  int idle_rounds = 0;  // rounds since a slot of this class was last busy
 };
 
-// Rounds a class without busy slots stays in the stepped set: a class that
-// comes and goes costs a graph capture each time, a class that stays costs
-// its (empty) launches every step.
-constexpr int kKeepIdleRounds = 4;
 // Longest round while no request waits for admission, in units of
 // max_round_steps (fewer host round trips; a new arrival waits at most one
 // round).
@@ -244,18 +241,13 @@ void scheduler(fsl_server* s) {
       }
     }
     if (running.empty()) continue;
-    // one round: the classes with busy slots plus those idle for fewer than
-    // kKeepIdleRounds rounds (an idle class's kernels return at once, which
-    // is cheaper than a new graph capture while classes come and go), as
-    // many steps as the nearest completion, at most max_round_steps (or a
-    // few times that while nothing waits for admission)
+    // one round: the classes with busy slots, as many steps as the nearest
+    // completion, at most max_round_steps (or a few times that while nothing
+    // waits for admission)
     std::vector<fsl::Group*> gl;
-    for (auto& kv : s->groups) {
-      SGroup& G = *kv.second;
-      G.idle_rounds = G.busy > 0 ? 0 : G.idle_rounds + 1;
-      if (!G.slots.empty() && G.idle_rounds <= kKeepIdleRounds) gl.push_back(&G.g);
-    }
-    if (gl != s->exec.groups) s->exec.groups = gl;
+    for (auto& kv : s->groups)
+      if (kv.second->busy > 0) gl.push_back(&kv.second->g);
+    s->exec.groups = gl;
     bool waiting;
     {
       std::lock_guard<std::mutex> lk(s->mu);
@@ -264,7 +256,7 @@ void scheduler(fsl_server* s) {
     int64_t n = s->cfg.max_round_steps * (waiting ? 1 : kQuietRoundFactor);
     for (Request* r : running) n = std::min(n, r->remaining);
     const double ta = s->now();
-    int rc = fsl::exec_step(s->exec, n);
+    int rc = fsl::exec_step_each(s->exec, n);
     std::vector<Request*> fin;
     std::vector<std::array<int, 4>> errs;
     if (rc == FSL_OK) {
