@@ -100,6 +100,14 @@ SlotLayout layout(const Params& P, int np_cap) {
   return L;
 }
 
+// Bytes of the spread field from which unbonded particles are taken in cell
+// order (particle_at).  A step with uniform particles, in memory order and in
+// cell order: 128^3 with 131,072 435 and 422 us, 160^3 with 200,000 925 and
+// 902, 200^3 with 100,000 1488 and 1486, 256^3 with 1,000,000 5433 and 4317.
+// (16-bead chains lose: 160^3 with 65,536 780 and 790, 256^3 with 524,288
+// 3690 and 3751.)
+constexpr double kOrderBytes = 48e6;
+
 bool factor_ok(int n) {
   if (n < 3) return false;
   const int ps[5] = {2, 3, 5, 7, 11};
@@ -262,6 +270,7 @@ int make_params(const fsl_config& c, int64_t np, Params& P) {
       P.skin = skin;
       P.vl_cut2 = (c.cutoff + skin) * (c.cutoff + skin);
       P.vl_half2 = 0.25 * skin * skin;
+      P.order = 24.0 * P.nc > kOrderBytes;
     }
   }
   P.eta = c.shearviscosity;

@@ -58,6 +58,7 @@ struct Params {
   // rc + skin at the reference positions qref, rebuilt when a particle has
   // moved more than skin / 2 since; nolist: no pair forces, no cell list
   int verlet, nolist;
+  int order;  // spread and interpolation take the particles in cell order (particle_at)
   double skin, vl_cut2, vl_half2;  // skin, (rc + skin)^2, (skin / 2)^2
   int has_extra;
   double cutoff, cutoff2, invcut2, soft_eps;
@@ -503,6 +504,21 @@ __device__ __forceinline__ bool quad_of(int blk, int np, long& e, int& a, int& q
   a = threadIdx.x & 3;
   qb = (threadIdx.x & 31) & ~3;
   return ((t & ~31L) >> 2) < np;
+}
+
+// The particle that place e of a particle launch takes.  With P.order the
+// places follow the cell list of the last Verlet rebuild at q: on grids whose
+// spread field does not stay in the L2, particles without order in memory
+// touch the whole field at any time, and cell order keeps the blocks in
+// flight within a few planes of it.  Bonded instances keep the order in
+// memory: beads of a chain follow each other there, and their warps share
+// stencil nodes.  Which place takes a particle changes no sum (the list may
+// be many steps old: it only has to be a permutation).
+__device__ __forceinline__ int particle_at(const Rep& R, long e) {
+  if (!R.P.order || R.P.bonded) return (int)e;
+  const int i = R.sorted[e];
+  // a build that gave up leaves stale entries (the error word says so)
+  return (unsigned)i < (unsigned)R.P.np ? i : 0;
 }
 
 // Launch kinds of the particle kernels (256-thread blocks): threads per

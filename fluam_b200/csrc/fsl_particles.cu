@@ -1376,7 +1376,7 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_spread(FSL_KARGS, int drift
   const bool on = e < np;  // lanes past the end join the shuffles only
   // cell order on the cell-list path (a list the step has just built)
   const bool by_cell = ordered && !P.verlet && !P.nolist;
-  const int i = on ? (by_cell ? cell_list(R, drift == 1).sorted[e] : (int)e) : 0;
+  const int i = on ? (by_cell ? cell_list(R, drift == 1).sorted[e] : particle_at(R, e)) : 0;
   bool sat = false;
   QuadStencil<KN> S;
   {
@@ -1973,7 +1973,7 @@ __global__ void k_interp_update(FSL_KARGS, int stage, int cached) {
   const int np = P.np;
   if (!quad_of(blk, np, e, a, qb)) return;
   const bool on = e < np;
-  const int i = on ? (int)e : 0;
+  const int i = on ? particle_at(R, e) : 0;
   const double* qpos = stage == 1 ? R.q : R.qp;
   double* qout = stage == 1 ? R.qp : R.q;
   QuadStencil<KN> S;
