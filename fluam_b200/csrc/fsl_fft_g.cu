@@ -223,7 +223,8 @@ __device__ __forceinline__ void gsecond(const GAxis& A, int t, const V* ex, cons
         [&](int b, V v) { emit(a + A.f[0] * b, v); });
 }
 
-// A whole line by A.t threads.  Output a of the first stage's thread t waits
+// A whole line by A.t threads (two stages that emit elsewhere than to the
+// other buffer need only b0).  Output a of the first stage's thread t waits
 // at pos(a, t) (two stages), point i between more stages at at(i).  Two
 // buffers; emit(f, value, other) gets the one that the last stage does not
 // read.  All threads of the block call this; `on` ones work.  The caller
@@ -711,7 +712,7 @@ struct GPlan {
   // single axes
   GLines lx, ly;
   int x_threads = 0, y_threads = 0, x_size = 0, y_size = 0;
-  size_t s_x = 0, s_y = 0;
+  size_t s_x = 0, s_xi = 0, s_y = 0;
   GZ z;
   int z_threads = 0, z_size = 0;
   size_t s_z = 0;
@@ -846,6 +847,10 @@ bool g_build(GPlan* g, int optin) {
       g->s_x = (size_t)es * (g->mx + 2 * (size_t)g->x_size);
       if (x.nl == 1 || g->s_x <= 100 * 1024) break;
     }
+    // the inverse and the y passes emit to global memory: one buffer where
+    // there are two stages, which doubles the blocks an SM holds (256^3: y
+    // 118 us a pass, inverse x 133 us with two buffers)
+    g->s_xi = mx_ ? g->s_x : (size_t)es * (g->mx + (size_t)ax.f[0] * x.pitch);
     g->x_threads = round_to(x.nl * ax.t, 32);
     GLines& y = g->ly;
     y = GLines{};
@@ -853,12 +858,12 @@ bool g_build(GPlan* g, int optin) {
     y.tw = g->tw[1];
     for (y.nl = std::max(1, std::min(g->mxh, cap / 2 / ay.t));; y.nl = std::max(1, y.nl / 2)) {
       g->y_size = y.nl * g->my;
-      g->s_y = (size_t)es * (g->my + 2 * (size_t)g->y_size);
+      g->s_y = (size_t)es * (g->my + (my_ ? 2 : 1) * (size_t)g->y_size);
       if (y.nl == 1 || g->s_y <= 100 * 1024) break;
     }
     g->y_threads = round_to(y.nl * ay.t, 32);
     if (g->x_threads > cap || g->y_threads > cap || !g_allow((const void*)GK<V>::xf(mx_), g->s_x, optin) ||
-        !g_allow((const void*)GK<V>::xi(mx_), g->s_x, optin) || !g_allow((const void*)GK<V>::yf(my_), g->s_y, optin) ||
+        !g_allow((const void*)GK<V>::xi(mx_), g->s_xi, optin) || !g_allow((const void*)GK<V>::yf(my_), g->s_y, optin) ||
         !g_allow((const void*)GK<V>::yi(my_), g->s_y, optin))
       return false;
   }
@@ -930,7 +935,7 @@ int g_inverse(const Batch& B, const GPlan* g, int ncomp, int pred, double scale,
   GLines x = g->lx;
   x.scale = scale;
   const long np = ((long)ncomp * g->my * g->mz + 1) / 2;
-  fsl_launch(GK<V>::xi(g->ax.ns > 2), dim3((unsigned)((np + x.nl - 1) / x.nl), B.nrep), g->x_threads, g->s_x, s, a, x,
+  fsl_launch(GK<V>::xi(g->ax.ns > 2), dim3((unsigned)((np + x.nl - 1) / x.nl), B.nrep), g->x_threads, g->s_xi, s, a, x,
              g->x_size);
   return 2;
 }
