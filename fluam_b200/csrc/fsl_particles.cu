@@ -786,6 +786,28 @@ void lists_autotune(const Batch& B, cudaStream_t s, float us[2]) {
   cudaGetLastError();
 }
 
+// The force over r of a pair within the cutoff.
+__device__ __forceinline__ double pair_factor(const Params& P, const Rep& R, double r2) {
+  return P.pair == 1 ? (double)tex_linear(R.ljtab, kLjTableSize, (float)(r2 * P.invcut2))
+                     : 2.0 * P.soft_eps / P.cutoff * (rsqrt(r2) - 1.0 / P.cutoff);
+}
+
+// The bonds of particle i that lane a of its quad takes.
+__device__ __forceinline__ void quad_bonds(const Rep& R, const double* __restrict__ q, int np, int i, int a, double rx, double ry,
+                                           double rz, double& fx, double& fy, double& fz) {
+  int nb = R.bpp_cnt[i], off = R.bpp_off[i];
+  for (int j = a; j < nb; j += 4) {
+    const int idx = R.bpp_idx[off + j];
+    bond_force(rx, ry, rz, q[idx], q[np + idx], q[2 * np + idx], R.bpp_k[off + j], R.bpp_r0[off + j], fx, fy, fz);
+  }
+  nb = R.bfp_cnt[i];
+  off = R.bfp_off[i];
+  for (int j = a; j < nb; j += 4) {
+    const double* p = R.bfp_xyz + 3 * (off + j);
+    bond_force(rx, ry, rz, p[0], p[1], p[2], R.bfp_k[off + j], R.bfp_r0[off + j], fx, fy, fz);
+  }
+}
+
 // The pair (Verlet list, or the 27 cells of the current cell list in cell
 // mode) and bonded force on particle i by its quad: lane a takes list
 // entries and bonds a, a + 4, ...; the partial forces are summed in a fixed
@@ -800,25 +822,7 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
   fx = 0.0;
   fy = 0.0;
   fz = 0.0;
-  if (P.bonded && on) {
-    int nb = R.bpp_cnt[i], off = R.bpp_off[i];
-    for (int j = a; j < nb; j += 4) {
-      const int idx = R.bpp_idx[off + j];
-      bond_force(rx, ry, rz, q[idx], q[np + idx], q[2 * np + idx], R.bpp_k[off + j], R.bpp_r0[off + j],
-                 fx, fy, fz);
-    }
-    nb = R.bfp_cnt[i];
-    off = R.bfp_off[i];
-    for (int j = a; j < nb; j += 4) {
-      const double* p = R.bfp_xyz + 3 * (off + j);
-      bond_force(rx, ry, rz, p[0], p[1], p[2], R.bfp_k[off + j], R.bfp_r0[off + j], fx, fy, fz);
-    }
-  }
-  const double c1 = 2.0 * P.soft_eps / P.cutoff, c2 = 1.0 / P.cutoff;
-  // the force over r of a pair within the cutoff
-  auto pair = [&](double r2) {
-    return P.pair == 1 ? (double)tex_linear(R.ljtab, kLjTableSize, (float)(r2 * P.invcut2)) : c1 * (rsqrt(r2) - c2);
-  };
+  if (P.bonded && on) quad_bonds(R, q, np, i, a, rx, ry, rz, fx, fy, fz);
   if (P.verlet && on && cell_mode) {
     // the 27 neighbour cells of the current cell list, lanes taking cells
     // a, a + 4, ...
@@ -837,7 +841,7 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
         const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rxij, rxij), __dmul_rn(ryij, ryij)),
                                     __dmul_rn(rzij, rzij));
         if (j == i || r2 >= P.cutoff2 || r2 == 0.0) continue;
-        const double f = pair(r2);
+        const double f = pair_factor(P, R, r2);
         fx += f * rxij;
         fy += f * ryij;
         fz += f * rzij;
@@ -853,10 +857,64 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
       const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rxij, rxij), __dmul_rn(ryij, ryij)),
                                   __dmul_rn(rzij, rzij));
       if (r2 >= P.cutoff2 || r2 == 0.0) continue;
-      const double f = pair(r2);
+      const double f = pair_factor(P, R, r2);
       fx += f * rxij;
       fy += f * ryij;
       fz += f * rzij;
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    fx += __shfl_xor_sync(0xffffffffu, fx, o);
+    fy += __shfl_xor_sync(0xffffffffu, fy, o);
+    fz += __shfl_xor_sync(0xffffffffu, fz, o);
+  }
+}
+
+// The same by a whole warp for one particle: a lane per list entry, whose
+// force factor and separations then go to the quads' lanes, which add them in
+// the order of quad_force_vl (entries a, a + 4, ... by lane a), so the sums
+// have its bits.  (All eight quads walking the list alike took the chain of
+// every fourth entry's loads: 33 us for a spread of 8,000 particles with 25
+// neighbours each.)
+__device__ __forceinline__ void warp_force_vl(const Params& P, const Rep& R, int i, int which, bool cell_mode, double& fx, double& fy,
+                                              double& fz) {
+  const int lane = threadIdx.x & 31, a = lane & 3;
+  const int n = P.verlet && !cell_mode ? R.vl_cnt[i] : 0;  // uniform
+  if (n <= 8) {
+    quad_force_vl(P, R, i, a, which, true, cell_mode, fx, fy, fz);
+    return;
+  }
+  const int np = P.np;
+  const double* __restrict__ q = which ? R.qp : R.q;
+  const double rx = q[i], ry = q[np + i], rz = q[2 * np + i];
+  fx = 0.0;
+  fy = 0.0;
+  fz = 0.0;
+  if (P.bonded) quad_bonds(R, q, np, i, a, rx, ry, rz, fx, fy, fz);
+  for (int base = 0; base < n; base += 32) {
+    const int k = base + lane;
+    double x = 0.0, y = 0.0, z = 0.0, f = 0.0;
+    bool on = k < n;
+    if (on) {
+      const int j = R.vl_idx[(size_t)k * np + i];
+      x = minimage(rx - q[j], P.invlx, P.lx);
+      y = minimage(ry - q[np + j], P.invly, P.ly);
+      z = minimage(rz - q[2 * np + j], P.invlz, P.lz);
+      const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+      on = !(r2 >= P.cutoff2 || r2 == 0.0);
+      if (on) f = pair_factor(P, R, r2);
+    }
+    const unsigned have = __ballot_sync(0xffffffffu, on);
+    for (int m = 0; m < 32 && base + m < n; m += 4) {
+      if (!(have >> m & 15u)) continue;  // uniform
+      const double g = __shfl_sync(0xffffffffu, f, m + a), gx = __shfl_sync(0xffffffffu, x, m + a),
+                   gy = __shfl_sync(0xffffffffu, y, m + a), gz = __shfl_sync(0xffffffffu, z, m + a);
+      if (have >> (m + a) & 1u) {
+        fx += g * gx;
+        fy += g * gy;
+        fz += g * gz;
+      }
     }
   }
 #pragma unroll
@@ -1433,8 +1491,8 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_spread(FSL_KARGS, int drift
 // chain's latency.  Here a warp takes one particle: lane (f 3 + d) KN + k
 // computes node k of family f in dimension d, the nodes go round by shuffles,
 // and lane a + 4 b + 16 c0 handles the x node a, the y node b and the z nodes
-// c0, c0 + 2 of every component.  Forces are quad_force_vl's, taken by all
-// eight quads of the warp alike.  Same products, same integer sums, same
+// c0, c0 + 2 of every component.  Forces are quad_force_vl's
+// (warp_force_vl).  Same products, same integer sums, same
 // order of every FP32 and FP64 sum: the bits of the quad kernels.
 // Launches of at most this many quad blocks (64 particles each) take it: one
 // block per SM.  A step of 64^3 cells, 4-point kernel: 512 particles 127 us
@@ -1532,7 +1590,7 @@ __global__ void __launch_bounds__(kPartThreads) k_spread_wide(FSL_KARGS, int dri
     const double pos[3] = {qf[i], qf[np + i], qf[2 * np + i]};
     double val[3];
     if (own_forces) {
-      quad_force_vl(P, R, i, lane & 3, drift == 1 ? 1 : 0, true, cell_mode, val[0], val[1], val[2]);
+      warp_force_vl(P, R, i, drift == 1 ? 1 : 0, cell_mode, val[0], val[1], val[2]);
       if (lane == 0) {
         if (!isfinite(val[0]) || !isfinite(val[1]) || !isfinite(val[2])) set_err(R.err, 2);
         R.F[i] = val[0];

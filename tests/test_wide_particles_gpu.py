@@ -56,3 +56,29 @@ def test_batch_equals_alone(fsl, name):
             np.testing.assert_array_equal(b.forces(i), g.forces())
         g.close()
     b.close()
+
+
+@pytest.mark.parametrize("cutoff", [3.2, 5.0, 6.0])
+def test_lennard_jones_lists(fsl, cutoff):
+    """Lists of a few, a few dozen and (with the cells of a box of 24) nearly
+    64 entries, whose forces a warp takes entry by entry."""
+    m, L = (24, 24, 24), (24.0, 24.0, 24.0)
+    rng = np.random.default_rng(1)
+    counts = [1, 2, 33, 400] + [512] * 10
+    qs = []
+    for n in counts:
+        sites = rng.permutation(512)[:n]
+        s = np.stack([sites % 8, sites // 8 % 8, sites // 64])
+        qs.append((s + 0.5) * 3.0 - 12.0 + rng.uniform(-0.2, 0.2, s.shape))
+    cfgs = [fsl.make_config(m, L, eta=1.0, kT=0.01, dt=0.01, cutoff=cutoff, kernel=3, pair=fsl.PAIR_TABLE_LJ, seed=i) for i in range(len(qs))]
+    b = fsl.Batch(cfgs, qs)
+    b.step(3)
+    b.sync()
+    for i, (c, q) in enumerate(zip(cfgs, qs)):
+        g = fsl.StokesLimit(c, q)
+        g.step(3)
+        g.sync()
+        np.testing.assert_array_equal(b.positions(i), g.positions())
+        np.testing.assert_array_equal(b.forces(i), g.forces())
+        g.close()
+    b.close()
