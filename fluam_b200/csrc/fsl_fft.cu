@@ -18,6 +18,8 @@
 // The multiplier keeps Hermitian symmetry (the sign of sin(pi j/m) for
 // j > m/2 cancels between gradient and shift), so the real-to-complex form
 // equals the reference's Re(IFFT(...)) up to rounding.
+#include <cooperative_groups.h>
+
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -35,16 +37,24 @@ constexpr int kMaxMx = 825, kMaxMy = 875, kMaxMz = 588;
 constexpr int kMaxZCand = 6;
 constexpr int kMaxPCand = 4;
 
+struct WSrc;  // fsl_fft_reg.cuh
+
 struct FftPlan {
   float2 *twx = nullptr, *twy = nullptr, *twz = nullptr;  // exp(-2 pi i t / m)
   // sin(pi j / m); the kernel multiplies by the instance's 2/h, so one table
   // serves every instance of a size class whatever its box
   float *sx = nullptr, *sy = nullptr, *sz = nullptr;
   float2 *ex = nullptr, *ey = nullptr, *ez = nullptr;  // exp(+i pi j / m)
+  // the whole solve of a small cube in one launch (fsl_fft_cube.cuh), for a
+  // single instance; null for other extents
+  void (*cube)(Rep, const float2*, const float*, const float*, const float*, const float2*, const float2*, const float2*,
+               WSrc) = nullptr;
+  int cube_threads = 0;
+  size_t smem_cube = 0;
   GPlan* gen = nullptr;  // general passes (fsl_fft_g.cu), where the compiled ones do not serve both parts
   bool ok = false;
   // register-resident passes for compiled edges (null: not available)
-  void (*plane_fwd_r[2])(RepSrc, Rep, const float2*) = {};
+  void (*plane_fwd_r[2])(RepSrc, Rep, const float2*, WSrc) = {};
   void (*plane_inv_r[2])(RepSrc, Rep, const float2*) = {};
   void (*zsolve_r[2])(RepSrc, Rep, const float2*, const float*, const float*, const float*,
                       const float2*, const float2*, const float2*) = {};
@@ -56,6 +66,7 @@ struct FftPlan {
   void (*line_xi[2])(RepSrc, Rep, const float2*) = {};
   int line_lw = 0;          // lines per warp
   size_t smem_lines = 0;
+  bool plane_v = false;     // the plane passes are the 128 edge's (fsl_fft_v.cuh)
   bool use_lines = false;   // the five-pass schedule (picked by fft_autotune)
   float sched_us[2] = {};   // measured solve transform time: plane, lines
   int plane_pb = 0, plane_threads = 0;      // planes per block, threads per block
@@ -76,7 +87,7 @@ struct FftPlan {
   // arithmetic, another number of independent planes per block); the first
   // is the default, fft_autotune picks one
   struct PCand {
-    void (*fwd[2])(RepSrc, Rep, const float2*);
+    void (*fwd[2])(RepSrc, Rep, const float2*, WSrc);
     void (*inv[2])(RepSrc, Rep, const float2*);
     int pb, threads;
     size_t smem;
@@ -259,6 +270,7 @@ __global__ void k_wbuild4(FSL_KARGS, int nsets, double nfac, int clear) {
 #include "fsl_fft_reg.cuh"
 #include "fsl_fft_lines.cuh"
 #include "fsl_fft_v.cuh"
+#include "fsl_fft_cube.cuh"
 
 // ------------------------------------------------------------ host side ---
 static void use_pcand(FftPlan* fp, int i) {
@@ -316,6 +328,7 @@ static void pick_plane_r(FftPlan* fp) {
       c.inv[0] = k_plane_inv_v<false>;
       c.inv[1] = k_plane_inv_v<true>;
       c.smem = sizeof(float2) * (size_t)kVSmem;
+      fp->plane_v = true;
     }
   }
   use_pcand(fp, 0);
@@ -368,6 +381,14 @@ static void pick_z_r(FftPlan* fp) {
   if (fp->nzc == 1) use_zcand(fp, 0);
 }
 
+template <int N, int R, int T>
+static void pick_cube(FftPlan* fp) {
+  using C = CubeGeom<N, R, T>;
+  fp->cube = k_solve_cube<N, R, T>;
+  fp->cube_threads = C::THREADS;
+  fp->smem_cube = sizeof(float2) * C::SMEM;
+}
+
 // Register-pass shapes per edge: N = R x T; planes per block; z tiles.
 static void pick_register_kernels(const Params& P, FftPlan* fp) {
   if (P.mx == P.my) {
@@ -384,6 +405,13 @@ static void pick_register_kernels(const Params& P, FftPlan* fp) {
       case 88: pick_plane_r<88, 8, 11, 1>(fp); break;
       case 96: pick_plane_r<96, 24, 4, 1, 2>(fp); break;
       case 128: pick_plane_r<128, 16, 8, 1>(fp); break;
+      default: break;
+    }
+  }
+  if (P.mx == P.my && P.mx == P.mz) {
+    switch (P.mx) {
+      case 16: pick_cube<16, 16, 1>(fp); break;
+      case 24: pick_cube<24, 24, 1>(fp); break;
       default: break;
     }
   }
@@ -501,6 +529,7 @@ FftPlan* fft_plan_create(const Params& P) {
     if (kept) use_zcand(fp, 0);
     else fp->zsolve_r[0] = fp->zsolve_r[1] = nullptr;
   }
+  if (fp->cube && (sched_env() != 0 || !allow((const void*)fp->cube, fp->smem_cube))) fp->cube = nullptr;
   // the five-pass schedule needs the register plane shapes (the same
   // packing) and the register z pass; fft_autotune takes it where it is
   // faster, the plane schedule serves until then (and classes that are never
@@ -594,9 +623,39 @@ static void zsolve(const Batch& B, const FftPlan* fp, cudaStream_t s) {
                fp->sy, fp->sz, fp->ex, fp->ey, fp->ez);
 }
 
+// The whole solve of a single small cube by one cluster of blocks.
+static bool cube_serves(const Batch& B, const FftPlan* fp) { return B.one && fp && fp->cube; }
+
+static void cube_solve(const Batch& B, const FftPlan* fp, const WSrc& ws, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kCubeRanks);
+  cfg.blockDim = dim3(fp->cube_threads);
+  cfg.dynamicSmemBytes = fp->smem_cube;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = kCubeRanks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  cudaLaunchKernelEx(&cfg, fp->cube, *B.one, (const float2*)fp->twx, (const float*)fp->sx, (const float*)fp->sy,
+                     (const float*)fp->sz, (const float2*)fp->ex, (const float2*)fp->ey, (const float2*)fp->ez, ws);
+}
+
+// Whether the forward plane pass builds W itself: the plane schedule, but for
+// the 128 edge's kernels.
+static bool fused_w(const FftPlan* fp) { return fp->plane_fwd_r[0] && !fp->use_lines && !fp->plane_v; }
+
+bool solve_clears_field(const Batch& B, const FftPlan* fp) {
+  return B.prec != PREC_F64 && fp && (cube_serves(B, fp) || fused_w(fp));
+}
+
 // The register path's transforms and solve with the plan's schedule: the
 // plane kernels (3 launches) or the five passes of warp tasks.
-static void reg_transform(const Batch& B, const FftPlan* fp, cudaStream_t s, Prof& pr) {
+static void reg_transform(const Batch& B, const FftPlan* fp, cudaStream_t s, Prof& pr, const WSrc& ws = WSrc{1, 0, 0.0}) {
   const int nrep = B.nrep;
   if (fp->use_lines) {
     const long lines = 3L * B.mz * (B.mx / 2);
@@ -625,9 +684,9 @@ static void reg_transform(const Batch& B, const FftPlan* fp, cudaStream_t s, Pro
   const int tb = fp->plane_threads;
   pr.mark(s, "plane_fwd");
   if (B.one)
-    fsl_launch(fp->plane_fwd_r[1], gp, tb, fp->smem_plane_r, s, RepSrc{}, *B.one, fp->twx);
+    fsl_launch(fp->plane_fwd_r[1], gp, tb, fp->smem_plane_r, s, RepSrc{}, *B.one, fp->twx, ws);
   else
-    fsl_launch(fp->plane_fwd_r[0], gp, tb, fp->smem_plane_r, s, B.src(), Rep{}, fp->twx);
+    fsl_launch(fp->plane_fwd_r[0], gp, tb, fp->smem_plane_r, s, B.src(), Rep{}, fp->twx, ws);
   pr.mark(s, "zsolve");
   zsolve(B, fp, s);
   pr.mark(s, "plane_inv");
@@ -676,18 +735,20 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
     if (fp->zc_us[i] < fp->zc_us[best]) best = i;
   use_zcand(fp, best);
   // planes per block of the plane schedule: the whole transform timed per
-  // candidate, as the z tiles
+  // candidate, as the z tiles, with W built on the way in where the steps do
+  // (the spread field is zero between steps)
   if (fp->npc > 1 && pcand_env() < 0 && sched_env() != 2) {
     const bool lines = fp->use_lines;
     fp->use_lines = false;
     Prof none;
+    const WSrc ws = fused_w(fp) ? WSrc{0, 1, 1.0} : WSrc{1, 0, 0.0};
     for (int i = 0; i < fp->npc; ++i) fp->pc_us[i] = 1e30f;
     for (int round = 0; round < 3; ++round)
       for (int i = 0; i < fp->npc; ++i) {
         use_pcand(fp, i);
-        reg_transform(B, fp, s, none);  // warm-up
+        reg_transform(B, fp, s, none, ws);  // warm-up
         cudaEventRecord(e0, s);
-        for (int r = 0; r < 5; ++r) reg_transform(B, fp, s, none);
+        for (int r = 0; r < 5; ++r) reg_transform(B, fp, s, none, ws);
         cudaEventRecord(e1, s);
         float ms = 0.f;
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) ms = 1e9f;
@@ -751,6 +812,16 @@ void launch_solve(const Batch& B, FftPlan* fp, int nsets, double nfac, int w_giv
   Prof dummy;
   Prof& pr = prof ? *prof : dummy;
   const int nrep = B.nrep;
+  if (cube_serves(B, fp)) {
+    pr.mark(s, "solve");
+    cube_solve(B, fp, WSrc{w_given, nsets, nfac}, s);
+    pr.count(1);
+    return;
+  }
+  if (!w_given && fused_w(fp)) {
+    reg_transform(B, fp, s, pr, WSrc{0, nsets, nfac});
+    return;
+  }
   if (!w_given) {
     // W from the spread field and the noise; clears the spread field
     pr.mark(s, "wbuild");

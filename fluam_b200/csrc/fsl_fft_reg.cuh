@@ -220,6 +220,72 @@ __device__ __forceinline__ int line_freq(int t, int j, int b) {
   return line_a<R, T>(t, j) + R * b;
 }
 
+// Where a forward pass finds W: given in Rep::wbuf, or built on the way in
+// from the spread field, which is cleared behind the read, and the noise
+// divergence (the arithmetic of k_wbuild4).
+struct WSrc {
+  int given, nsets;
+  double nfac;
+};
+
+// W of U groups of four consecutive cells from indexes at(u) (multiples of
+// 4; negative: none), given to put(u, w).  All loads first: the stores that
+// clear the field would otherwise hold back the next group's loads, a memory
+// latency for each group.
+template <int U, class At, class Put>
+__device__ __forceinline__ void w_cells4(const Params& P, const Rep& R, const WSrc& ws, At&& at, Put&& put) {
+  if (ws.given) {
+    float4 w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (at(u) >= 0) w[u] = *reinterpret_cast<const float4*>(R.wbuf + at(u));
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (at(u) >= 0) put(u, w[u]);
+    return;
+  }
+  const float fac = (float)ws.nfac;
+  const float* D = R.ndiv + (ws.nsets > 1 ? 3 * (size_t)P.nc : 0);
+  float4 d[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (at(u) >= 0) d[u] = __ldg(reinterpret_cast<const float4*>(D + at(u)));
+  if (P.prec == PREC_FLOAT) {
+    const float fscale = (float)(1.0 / P.dV);
+    float* gf = reinterpret_cast<float*>(R.grid);
+    float4 g[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (at(u) >= 0) g[u] = *reinterpret_cast<const float4*>(gf + at(u));
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (at(u) < 0) continue;
+      *reinterpret_cast<float4*>(gf + at(u)) = make_float4(0.f, 0.f, 0.f, 0.f);
+      put(u, make_float4(w_float(g[u].x, fscale, fac, d[u].x), w_float(g[u].y, fscale, fac, d[u].y),
+                         w_float(g[u].z, fscale, fac, d[u].z), w_float(g[u].w, fscale, fac, d[u].w)));
+    }
+    return;
+  }
+  const float scale = (float)(kFixedInv / P.dV);
+  longlong2 ga[U], gb[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (at(u) < 0) continue;
+    const longlong2* gp = reinterpret_cast<const longlong2*>(R.grid + at(u));
+    ga[u] = gp[0];
+    gb[u] = gp[1];
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (at(u) < 0) continue;
+    longlong2* gp = reinterpret_cast<longlong2*>(R.grid + at(u));
+    gp[0] = make_longlong2(0, 0);
+    gp[1] = make_longlong2(0, 0);
+    put(u, make_float4(w_fixed(ga[u].x, scale, fac, d[u].x), w_fixed(ga[u].y, scale, fac, d[u].y),
+                       w_fixed(gb[u].x, scale, fac, d[u].z), w_fixed(gb[u].y, scale, fac, d[u].w)));
+  }
+}
+
 // Real-to-complex transform of whole xy planes (x then y), PB planes per
 // block, H * T threads per plane (H = N / 2).  x: the row pair (2p, 2p+1) is
 // one complex line; y: columns kx = 1 .. H-1 are complex lines and columns 0
@@ -227,7 +293,7 @@ __device__ __forceinline__ int line_freq(int t, int j, int b) {
 // Output: the half spectrum spec[comp][z][ky][kx], kx <= H.
 template <bool ONE, int N, int RR, int T, int PB>
 __global__ void __launch_bounds__(PB * (N / 2) * T)
-    k_plane_fwd_r(FSL_KARGS, const float2* __restrict__ twn) {
+    k_plane_fwd_r(FSL_KARGS, const float2* __restrict__ twn, const WSrc ws) {
   FSL_REP_AT(blockIdx.z);
   using G = LineGeom<RR, T>;
   constexpr int H = N / 2, TPP = H * T, LS = G::LS;
@@ -239,12 +305,24 @@ __global__ void __launch_bounds__(PB * (N / 2) * T)
   const int pl = blockIdx.x * PB + lp;  // comp * mz + z
   const bool live = pl < 3 * P.mz;
   const int comp = live ? pl / P.mz : 0, z = live ? pl - comp * P.mz : 0;
-  const float* W = R.wbuf + (size_t)comp * P.nc + (size_t)z * N * N;
+  const size_t at0 = (size_t)comp * P.nc + (size_t)z * N * N;  // the plane's first cell
+  static_assert(N % 4 == 0, "rows of whole groups of four cells");
   float2 v[RR];
   if constexpr (T == 1) {
     // stage the plane through shared memory so the global reads coalesce
     float* fb = reinterpret_cast<float*>(buf);
-    for (int i = r; i < N * N; i += TPP) fb[i + (i / N)] = live ? W[i] : 0.0f;  // row pitch N + 1
+    constexpr int U = 4;
+    for (int i = 4 * r; i < N * N; i += 4 * TPP * U)
+      w_cells4<U>(
+          P, R, ws, [&](int u) { const int j = i + 4 * TPP * u; return live && j < N * N ? (long)(at0 + j) : -1L; },
+          [&](int u, float4 w) {
+            const int j = i + 4 * TPP * u;
+            float* f = fb + j + j / N;  // row pitch N + 1
+            f[0] = w.x;
+            f[1] = w.y;
+            f[2] = w.z;
+            f[3] = w.w;
+          });
     __syncthreads();
     const int p = r;
 #pragma unroll
@@ -254,8 +332,8 @@ __global__ void __launch_bounds__(PB * (N / 2) * T)
 #pragma unroll
     for (int f = 0; f < N; ++f) buf[p * LS + f] = v[f];
   } else {
-    // The W planes come into the planes' buffers row by row (N floats at
-    // pitch PW = N + 4; rows, pitch and buffer starts are multiples of 16
+    // W built here goes into rows of PW = N + 4 floats.  A given W comes into
+    // the planes' buffers row by row (N floats at pitch PW; rows, pitch and buffer starts are multiples of 16
     // bytes) by bulk copies on the block's mbarrier (bounded wait), and the
     // x pass reads them from shared memory: at pitch N + 4 a warp load takes
     // two wavefronts (four at edge 32) where reading the rows from global
@@ -266,22 +344,34 @@ __global__ void __launch_bounds__(PB * (N / 2) * T)
                       plane_buf<N, RR, T>() % 2 == 0 && PB * N * kRowBytes < (1u << 20),
                   "row-wise bulk copies of the W planes");
     __shared__ __align__(8) unsigned long long s_bar;
-    if (threadIdx.x == 0) {
-      mbar_init(&s_bar, 1);
-      mbar_fence_init();
+    if (!ws.given) {
+      float* f = reinterpret_cast<float*>(buf);
+      constexpr int U = 4;
+      for (int i = 4 * r; i < N * N; i += 4 * TPP * U)
+        w_cells4<U>(
+            P, R, ws, [&](int u) { const int j = i + 4 * TPP * u; return live && j < N * N ? (long)(at0 + j) : -1L; },
+            [&](int u, float4 w) {
+              const int j = i + 4 * TPP * u;
+              *reinterpret_cast<float4*>(f + j / N * PW + j % N) = w;
+            });
+    } else {
+      if (threadIdx.x == 0) {
+        mbar_init(&s_bar, 1);
+        mbar_fence_init();
+      }
+      __syncthreads();
+      // blockIdx.x PB < 3 mz, so the block has at least one live plane
+      const int nlive = min(PB, 3 * P.mz - (int)blockIdx.x * PB);
+      if (threadIdx.x == 0) mbar_arrive_tx(&s_bar, kRowBytes * (unsigned)(N * nlive));
+      __syncthreads();
+      for (int i = threadIdx.x; i < N * nlive; i += blockDim.x) {
+        const int q = i / N, row = i - q * N;
+        const int plq = blockIdx.x * PB + q, cq = plq / P.mz, zq = plq - cq * P.mz;
+        bulk_load(reinterpret_cast<float*>(smem + N + q * plane_buf<N, RR, T>()) + row * PW,
+                  R.wbuf + (size_t)cq * P.nc + ((size_t)zq * N + row) * N, kRowBytes, &s_bar);
+      }
+      bulk_wait(&s_bar, R.err);
     }
-    __syncthreads();
-    // blockIdx.x PB < 3 mz, so the block has at least one live plane
-    const int nlive = min(PB, 3 * P.mz - (int)blockIdx.x * PB);
-    if (threadIdx.x == 0) mbar_arrive_tx(&s_bar, kRowBytes * (unsigned)(N * nlive));
-    __syncthreads();
-    for (int i = threadIdx.x; i < N * nlive; i += blockDim.x) {
-      const int q = i / N, row = i - q * N;
-      const int plq = blockIdx.x * PB + q, cq = plq / P.mz, zq = plq - cq * P.mz;
-      bulk_load(reinterpret_cast<float*>(smem + N + q * plane_buf<N, RR, T>()) + row * PW,
-                R.wbuf + (size_t)cq * P.nc + ((size_t)zq * N + row) * N, kRowBytes, &s_bar);
-    }
-    bulk_wait(&s_bar, R.err);
     __syncthreads();
     const float* fw = reinterpret_cast<const float*>(buf);  // this thread's plane
     const int p = r / T, t = r - p * T;

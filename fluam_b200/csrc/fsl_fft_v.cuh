@@ -70,9 +70,11 @@ __device__ __forceinline__ void v_line_b(const float2* lb, int t, int dir, float
   RDft<8>::run(out[1], dir);
 }
 
-// Forward: W plane (comp, z) -> half spectrum, as k_plane_fwd_r<128,16,8,1>.
+// Forward: W plane (comp, z) -> half spectrum, as k_plane_fwd_r<128,16,8,1>
+// (W is always given: built here, the pass took 119 us for two against 57 + 49
+// apart).
 template <bool ONE>
-__global__ void __launch_bounds__(512) k_plane_fwd_v(FSL_KARGS, const float2* __restrict__ twn) {
+__global__ void __launch_bounds__(512) k_plane_fwd_v(FSL_KARGS, const float2* __restrict__ twn, const WSrc) {
   FSL_REP_AT(blockIdx.z);
   constexpr int N = 128, H = 64;
   extern __shared__ __align__(16) float2 smem[];

@@ -844,7 +844,7 @@ void group_enqueue_step(Group& g) {
   // the field clear after a W build goes to the side stream, where its
   // blocks fill the SMs that the transforms leave idle; the W build then
   // only reads the field
-  const bool clear_fork = fork && !B.tiled && B.prec != PREC_F64;
+  const bool clear_fork = fork && !B.tiled && B.prec != PREC_F64 && !solve_clears_field(B, g.fft);
   auto solve = [&](int k, int nsets, double nfac) {
     launch_solve(B, g.fft, nsets, nfac, B.tiled, s, &pr, clear_fork ? g.ev_w[k] : nullptr);
     chk("solve");

@@ -799,6 +799,9 @@ void fft_tuning(const FftPlan* fp, FftTuning& out);
 // after that event and before the next spread.
 void launch_solve(const Batch& B, FftPlan* fp, int nsets, double nfac, int w_given, cudaStream_t s,
                   Prof* prof = nullptr, cudaEvent_t w_built = nullptr);
+// Whether launch_solve clears B's spread field itself, with or without
+// w_built.
+bool solve_clears_field(const Batch& B, const FftPlan* fp);
 // Zeroes the spread fields of B's instances (streaming stores).
 void launch_field_clear(const Batch& B, cudaStream_t s);
 }  // namespace fsl
