@@ -209,7 +209,8 @@ int fsl_set_positions(fsl_handle* h, const double* in) {
 int fsl_step_io(fsl_handle* h, const double* in, double* out) {
   if (!h || !in || !out) return errorf(FSL_E_ARG, "null argument");
   FSL_TRY(cudaSetDevice(h->exec.device));
-  if (!fsl::pinned_host(in) || !fsl::pinned_host(out)) {
+  void *din = nullptr, *dout = nullptr;
+  if (!fsl::pinned_host(in, &din) || !fsl::pinned_host(out, &dout)) {
     // pageable buffers: the copies stay outside the step's graph
     if (int rc = fsl_set_positions(h, in)) return rc;
     if (int rc = fsl_step(h, 1)) return rc;
@@ -219,9 +220,13 @@ int fsl_step_io(fsl_handle* h, const double* in, double* out) {
   g.io_in = in;
   g.io_out = out;
   g.io_bytes = sizeof(double) * 3 * (size_t)params(h).np;
+  g.io_kernels = din && dout && params(h).np <= fsl::kIoKernelNp;
+  g.io_in_dev = (const double*)din;
+  g.io_out_dev = (double*)dout;
   const int rc = fsl::exec_step(h->exec, 1);
   g.io_in = nullptr;
   g.io_out = nullptr;
+  g.io_kernels = false;
   if (rc) return rc;
   FSL_TRY(cudaStreamSynchronize(h->exec.stream));
   return FSL_OK;

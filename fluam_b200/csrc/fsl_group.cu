@@ -830,7 +830,10 @@ void group_enqueue_step(Group& g) {
   // memory beside the noise (which reads no position), then the Verlet-list
   // check of fsl_set_positions
   if (g.io_wait) cudaStreamWaitEvent(s, g.io_wait, 0);
-  if (g.io_in && !g.slots.empty()) {
+  if (g.io_in && g.io_kernels) {
+    launch_io_in(g.slots[0]->r, g.io_in_dev, s);
+    chk("positions in");
+  } else if (g.io_in && !g.slots.empty()) {
     cudaMemcpyAsync(g.slots[0]->r.q, g.io_in, g.io_bytes, cudaMemcpyHostToDevice, s);
     launch_moved_check(g.slots[0]->r, s);
     chk("positions in");
@@ -856,6 +859,12 @@ void group_enqueue_step(Group& g) {
   };
   auto join_clear = [&](int k) {
     if (clear_fork) cudaStreamWaitEvent(s, g.ev_c[k], 0);
+  };
+  // the end of the step: its counter, with the positions out of a small
+  // input/output step
+  auto count_step = [&]() {
+    if (g.io_out && g.io_kernels) launch_io_out(g.slots[0]->r, g.io_out_dev, s);
+    else launch_step_counter(B, s);
   };
   auto observe = [&]() {
     if (!g.key.observe) return;
@@ -883,7 +892,7 @@ void group_enqueue_step(Group& g) {
     chk("substep 2");
     pr.count(4 + nl);
     pr.mark(s, "counter");
-    launch_step_counter(B, s);
+    count_step();
     chk("counter");
     pr.count(1);
     pr.mark(s, nullptr);
@@ -907,12 +916,11 @@ void group_enqueue_step(Group& g) {
     launch_q2_solve(B, fft_general(g.fft), s, &pr);
     chk("solve");
     pr.mark(s, "q2_update");
-    launch_q2_update(B, 1, s);
-    launch_q2_update(B, 2, s);
+    pr.count(launch_q2_update(B, 1, s));
+    pr.count(launch_q2_update(B, 2, s));
     chk("update");
-    pr.count(2 * pk);
     pr.mark(s, "counter");
-    launch_step_counter(B, s);
+    count_step();
     chk("counter");
     pr.count(1);
     pr.mark(s, nullptr);
@@ -948,7 +956,7 @@ void group_enqueue_step(Group& g) {
     pr.count(pk);
     observe();
     pr.mark(s, "counter");
-    launch_step_counter(B, s);
+    count_step();
     chk("counter");
     pr.count(1);
     join_clear(0);
@@ -1025,7 +1033,7 @@ void group_enqueue_step(Group& g) {
   pr.count(pk);
   observe();
   pr.mark(s, "counter");
-  launch_step_counter(B, s);
+  count_step();
   chk("counter");
   pr.count(1);
   join_clear(1);
@@ -1068,12 +1076,13 @@ void exec_drop_graph(Exec& e) {
   e.shape.clear();
 }
 
-bool pinned_host(const void* p) {
+bool pinned_host(const void* p, void** dev) {
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
+  if (dev) *dev = a.devicePointer;
   return a.type == cudaMemoryTypeHost;
 }
 
@@ -1177,7 +1186,7 @@ void exec_enqueue_groups(Exec& e) {
     group_enqueue_step(g);
     e.launches_per_step = g.launches;
     // the positions after the step of an input/output step
-    if (g.io_out && !g.slots.empty())
+    if (g.io_out && !g.io_kernels && !g.slots.empty())
       cudaMemcpyAsync(g.io_out, g.slots[0]->r.q, g.io_bytes, cudaMemcpyDeviceToHost, e.stream);
     return;
   }

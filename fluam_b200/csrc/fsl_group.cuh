@@ -121,6 +121,11 @@ struct Group {
   const double* io_in = nullptr;
   double* io_out = nullptr;
   size_t io_bytes = 0;
+  // small instances: kernels read and write the host memory through its
+  // device addresses (launch_io_in, launch_io_out)
+  bool io_kernels = false;
+  const double* io_in_dev = nullptr;
+  double* io_out_dev = nullptr;
   // an input/output step of a batch: the step's main branch waits for this
   // event (the inputs copied in and scattered on the Exec's io stream)
   // after forking its noise
@@ -168,8 +173,8 @@ struct Exec {
 };
 
 // Whether p is page-locked host memory (a copy from or to it can be a node
-// of a CUDA graph).
-bool pinned_host(const void* p);
+// of a CUDA graph); dev: its address on the device (null: not mapped).
+bool pinned_host(const void* p, void** dev = nullptr);
 
 int exec_init(Exec& e, int device);
 void exec_destroy(Exec& e);

@@ -741,6 +741,12 @@ void launch_reset_lists(const Rep& r, cudaStream_t s);
 // After positions were replaced from the host: flag a Verlet-list rebuild if
 // a particle moved more than skin / 2 from its reference position.
 void launch_moved_check(const Rep& r, cudaStream_t s);
+// The ends of an input/output step of at most kIoKernelNp particles: q from
+// the device address `in` of page-locked host memory with the check of
+// launch_moved_check; q to `out` with the step counter.
+constexpr int kIoKernelNp = 16384;
+void launch_io_in(const Rep& r, const double* in, cudaStream_t s);
+void launch_io_out(const Rep& r, double* out, cudaStream_t s);
 // FP64 observables of every instance with P.observe (end of a step)
 void launch_observe(const Batch& B, cudaStream_t s);
 // The FP64 form (fsl_fp64.cu); the launchers above hand a class of that

@@ -566,6 +566,41 @@ void launch_moved_check(const Rep& r, cudaStream_t s) {
   k_moved_check<<<b, 256, 0, s>>>(r);
 }
 
+// The ends of a small instance's input/output step: positions read from and
+// written to page-locked host memory by kernels (the first also takes the
+// check of launch_moved_check, the last the step counter), instead of copy
+// nodes beside them: each copy engine node costs the step's chain 4 us.
+__global__ void k_io_in(const __grid_constant__ Rep R, const double* __restrict__ in) {
+  fsl_pdl_enter();
+  const Params& P = R.P;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.np; i += gridDim.x * blockDim.x) {
+    double d2 = 0.0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const size_t k = (size_t)d * P.np + i;
+      const double x = in[k];
+      R.q[k] = x;
+      if (P.verlet) d2 += (x - R.qref[k]) * (x - R.qref[k]);
+    }
+    if (P.verlet && d2 > P.vl_half2) R.vl_flag[0] = *R.t + 1;
+  }
+}
+
+__global__ void k_io_out(const __grid_constant__ Rep R, double* __restrict__ out) {
+  fsl_pdl_enter();
+  const long n3 = 3l * R.P.np;
+  for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n3; k += (long)gridDim.x * blockDim.x) out[k] = R.q[k];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *R.t += 1;
+}
+
+void launch_io_in(const Rep& r, const double* in, cudaStream_t s) {
+  if (r.P.np > 0) fsl_launch(k_io_in, dim3((unsigned)(r.P.np + 255) / 256), dim3(256), 0, s, r, in);
+}
+
+void launch_io_out(const Rep& r, double* out, cudaStream_t s) {
+  fsl_launch(k_io_out, dim3((unsigned)std::max(1, (3 * r.P.np + 255) / 256)), dim3(256), 0, s, r, out);
+}
+
 // ----------------------------------------------- single-launch list build ---
 // The cell list (and the Verlet list) of one instance in one cooperative
 // launch: the phases of the kernels above separated by grid barriers, so a
