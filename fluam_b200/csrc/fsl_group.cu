@@ -912,7 +912,6 @@ void group_enqueue_step(Group& g) {
     join_noise();
     launch_q2_field(B, s, &pr);
     chk("spread");
-    pr.count(2 + pk);
     launch_q2_solve(B, fft_general(g.fft), s, &pr);
     chk("solve");
     pr.mark(s, "q2_update");

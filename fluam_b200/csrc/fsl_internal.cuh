@@ -763,7 +763,7 @@ void launch_inc_load(const Batch& B, cudaStream_t s);
 void launch_q2_forces(const Batch& B, cudaStream_t s);
 void launch_q2_field(const Batch& B, cudaStream_t s, Prof* prof);
 void launch_q2_solve(const Batch& B, const GPlan* g, cudaStream_t s, Prof* prof);
-void launch_q2_update(const Batch& B, int stage, cudaStream_t s);
+int launch_q2_update(const Batch& B, int stage, cudaStream_t s);  // kernels launched
 
 // Transforms of any 2,3,5,7,11-smooth extents (fsl_fft_g.cu), in the
 // precision of the class: the real field (Rep::wbuf or w64) of ncomp

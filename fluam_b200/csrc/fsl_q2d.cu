@@ -398,7 +398,10 @@ void launch_q2_field(const Batch& B, cudaStream_t s, Prof* prof) {
   if (prof) prof->mark(s, "q2_spread");
   FSL_GO(k_q2_zero, dim3(bc, B.nrep), tb, 0, s, B);
   if (B.max_np > 0) FSL_GO(k_q2_spread, part_blocks(B, KIND_T32), kPartThreads, 0, s, B);
-  FSL_GO(k_q2_shear, dim3(bc, B.nrep), tb, 0, s, B);
+  // (a single instance is part of the captured step's shape)
+  const bool shear = !(B.one && B.one->P.q2_shear == 0.0);
+  if (shear) FSL_GO(k_q2_shear, dim3(bc, B.nrep), tb, 0, s, B);
+  if (prof) prof->count(1 + (B.max_np > 0 ? 1 : 0) + (shear ? 1 : 0));
 }
 
 void launch_q2_solve(const Batch& B, const GPlan* g, cudaStream_t s, Prof* prof) {
@@ -415,9 +418,10 @@ void launch_q2_solve(const Batch& B, const GPlan* g, cudaStream_t s, Prof* prof)
   if (prof) prof->count(n + 1);
 }
 
-void launch_q2_update(const Batch& B, int stage, cudaStream_t s) {
-  if (B.max_np == 0) return;
+int launch_q2_update(const Batch& B, int stage, cudaStream_t s) {
+  if (B.max_np == 0 || (stage == 2 && B.one && !B.one->P.q2_pc)) return 0;
   FSL_GO(k_q2_update, part_blocks(B, KIND_T32), kPartThreads, 0, s, B, stage);
+  return 1;
 }
 
 }  // namespace fsl
