@@ -213,7 +213,8 @@ __global__ void k_field_clear(FSL_KARGS) {
   const size_t bytes = (size_t)3 * P.nc * (P.prec == PREC_FLOAT ? 4 : 8);
   float4* q = reinterpret_cast<float4*>(R.grid);
   const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < bytes / 16; i += (size_t)gridDim.x * blockDim.x)
+  // (the buffer is padded to 256 bytes: a last partial group is cleared whole)
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (bytes + 15) / 16; i += (size_t)gridDim.x * blockDim.x)
     __stcs(q + i, z);
 }
 
