@@ -132,12 +132,13 @@ def stage_bytes(name, P):
         # force spread + the drift test (reference mode: the drift spreads
         # cancel and are skipped except at stencil changes)
         "spread_rfd": part + 2 * touched + 36 * npart,
-        # int64 field read + cleared, divergence of the noise read, W written
-        # (the per-stage pass keeps one stream, so its W build clears the
-        # field itself; the headline pass clears it on the side stream)
+        # (five-pass schedule) int64 field read + cleared, divergence of the
+        # noise read, W written
         "wbuild": 24 * nc + 24 * nc + 12 * nc + 12 * nc,
         "field_clear": 24 * nc,
-        "plane_fwd": 12 * nc + spec,               # W read, half spectrum written
+        # W built on the way in: int64 field read and cleared, divergence of
+        # the noise read, half spectrum written
+        "plane_fwd": 24 * nc + 24 * nc + 12 * nc + spec,
         "plane_inv": spec + 12 * nc,
         "fft_x": 12 * nc + spec,                   # line schedule: x forward or inverse
         "fft_y": 2 * spec,

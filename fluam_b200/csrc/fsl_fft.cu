@@ -6,7 +6,8 @@
 // doubleComplexToDoubleNormalized).  The reference runs 3 + 3 cuFFT Z2Z
 // transforms and 5 elementwise passes per solve in FP64; here the transform is
 // a hand-written FP32 one done as passes over the half spectrum:
-//   k_wbuild    builds W from the fixed-point spread field and the noise;
+//   k_wbuild    builds W from the fixed-point spread field and the noise (the
+//               compiled plane passes build it on the way in);
 //   plane fwd   2-D real-to-complex transform of whole xy planes;
 //   z solve     transforms along z, applies the spectral multiplier to all
 //               three components of each mode, and transforms back along z;
@@ -66,7 +67,6 @@ struct FftPlan {
   void (*line_xi[2])(RepSrc, Rep, const float2*) = {};
   int line_lw = 0;          // lines per warp
   size_t smem_lines = 0;
-  bool plane_v = false;     // the plane passes are the 128 edge's (fsl_fft_v.cuh)
   bool use_lines = false;   // the five-pass schedule (picked by fft_autotune)
   float sched_us[2] = {};   // measured solve transform time: plane, lines
   int plane_pb = 0, plane_threads = 0;      // planes per block, threads per block
@@ -329,7 +329,6 @@ static void pick_plane_r(FftPlan* fp) {
       c.inv[0] = k_plane_inv_v<false>;
       c.inv[1] = k_plane_inv_v<true>;
       c.smem = sizeof(float2) * (size_t)kVSmem;
-      fp->plane_v = true;
     }
   }
   use_pcand(fp, 0);
@@ -646,9 +645,8 @@ static void cube_solve(const Batch& B, const FftPlan* fp, const WSrc& ws, cudaSt
                      (const float*)fp->sz, (const float2*)fp->ex, (const float2*)fp->ey, (const float2*)fp->ez, ws);
 }
 
-// Whether the forward plane pass builds W itself: the plane schedule, but for
-// the 128 edge's kernels.
-static bool fused_w(const FftPlan* fp) { return fp->plane_fwd_r[0] && !fp->use_lines && !fp->plane_v; }
+// Whether the forward plane pass builds W itself: the plane schedule.
+static bool fused_w(const FftPlan* fp) { return fp->plane_fwd_r[0] && !fp->use_lines; }
 
 bool solve_clears_field(const Batch& B, const FftPlan* fp) {
   return B.prec != PREC_F64 && fp && (cube_serves(B, fp) || fused_w(fp));

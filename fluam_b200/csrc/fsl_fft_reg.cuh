@@ -619,8 +619,14 @@ __global__ void __launch_bounds__(PB * (N / 2) * T)
 
 // z transform, Stokes solve of every mode, inverse z transform, for a tile
 // of KX kx values by KY ky values (all three components).  Line
-// l = (kyl * 3 + comp) * KX + kxl; thread r = t * nlines + l.  The solve is
-// the multiplier of k_zsolve.
+// l = (kyl * 3 + comp) * KX + kxl; thread r = t * nlines + l.  The solve:
+//   W'_a = W_a e^{-i pi j_a/m_a};  G2 = |g|^2, g_a = 2/h_a sin(pi j_a/m_a)
+//   V'_a = (W'_a - g_a (g.W')/G2) / (eta G2);  v_a = V'_a e^{+i pi j_a/m_a}/nc
+// and v = 0 for the zero mode (src/stokesLimitFunctions.cu:2399-2451 with the
+// shifts of src/realToComplex.cu:263-303 and the 1/ncells of :40-59).  (Edge
+// 256 bounded to 80 registers for two blocks per SM: 183 against 228 us alone,
+// but the step of 256^3 4613 against 4372 us, because the side stream's kernels
+// no longer find room beside it.)
 template <bool ONE, int MZ, int RR, int T, int KX, int KY>
 __global__ void __launch_bounds__(3 * KX * KY * T)
     k_zsolve_r(FSL_KARGS, const float2* __restrict__ twn, const float* __restrict__ sx,

@@ -70,11 +70,11 @@ __device__ __forceinline__ void v_line_b(const float2* lb, int t, int dir, float
   RDft<8>::run(out[1], dir);
 }
 
-// Forward: W plane (comp, z) -> half spectrum, as k_plane_fwd_r<128,16,8,1>
-// (W is always given: built here, the pass took 119 us for two against 57 + 49
-// apart).
+// Forward: W plane (comp, z), given or built on the way in, -> half spectrum,
+// as k_plane_fwd_r<128,16,8,1>.  With W built here the pass takes 37 us at
+// 128^3 where it took 25, without the W build's 16 and the field clear's 9.
 template <bool ONE>
-__global__ void __launch_bounds__(512) k_plane_fwd_v(FSL_KARGS, const float2* __restrict__ twn, const WSrc) {
+__global__ void __launch_bounds__(512, 2) k_plane_fwd_v(FSL_KARGS, const float2* __restrict__ twn, const WSrc ws) {
   FSL_REP_AT(blockIdx.z);
   constexpr int N = 128, H = 64;
   extern __shared__ __align__(16) float2 smem[];
@@ -85,17 +85,21 @@ __global__ void __launch_bounds__(512) k_plane_fwd_v(FSL_KARGS, const float2* __
   const bool live = pl < 3 * P.mz;
   const int comp = live ? pl / P.mz : 0, z = live ? pl - comp * P.mz : 0;
   v_twiddles(twt, twn);
-  // the real plane, 16-byte loads into rows of kVR floats (ordinary loads:
-  // measured faster here than bulk row copies or per-thread async copies)
+  // the real plane, 16-byte loads into rows of kVR floats (of a given W,
+  // ordinary loads measured faster here than bulk row copies or per-thread
+  // async copies)
   float* fb = reinterpret_cast<float*>(buf);
   {
-    const float4* W4 = reinterpret_cast<const float4*>(R.wbuf + (size_t)comp * P.nc + (size_t)z * N * N);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int i = r + 512 * j, row = i >> 5, x4 = i & 31;
-      const float4 w = live ? W4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(fb + row * kVR + 4 * x4) = w;
-    }
+    const size_t at0 = (size_t)comp * P.nc + (size_t)z * N * N;
+    constexpr int U = 2;  // (64 registers: two blocks per SM)
+#pragma unroll 1
+    for (int j = 0; j < 8; j += U)
+      w_cells4<U>(
+          P, R, ws, [&](int u) { return live ? (long)(at0 + 4 * (r + 512 * (j + u))) : -1L; },
+          [&](int u, float4 w) {
+            const int i = r + 512 * (j + u);
+            *reinterpret_cast<float4*>(fb + (i >> 5) * kVR + 4 * (i & 31)) = w;
+          });
   }
   __syncthreads();
   // x pass: line p = rows (2p, 2p+1) as one complex line, lane t
