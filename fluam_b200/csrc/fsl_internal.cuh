@@ -127,15 +127,18 @@ __host__ __device__ inline uint4 philox4x32_10(uint4 c, const PhiloxKeys& K) {
   return c;
 }
 
+// (2 (w >> 9) + 1) 2^-24: the 23 bits as the fraction of a float in [1, 2),
+// less 1 - 2^-24; every step is exact (an integer-to-float conversion would
+// take the special-function pipe that the logarithms, roots and sines need).
+__device__ __forceinline__ float philox_uniform(uint32_t w) {
+  return __uint_as_float(0x3f800000u | (w >> 9)) - __uint_as_float(0x3f7fffffu);
+}
+
 // The four normal deviates of one Philox output r.  Word w becomes the
 // uniform (2 (w >> 9) + 1) 2^-24 in (0,1), exact in FP32; Box-Muller on the
 // pairs (u0,u1) and (u2,u3).
 __device__ inline float4 philox_box_muller(uint4 r) {
-  const float s24 = 5.9604644775390625e-08f;  // 2^-24
-  float u0 = (float)(2u * (r.x >> 9) + 1u) * s24;
-  float u1 = (float)(2u * (r.y >> 9) + 1u) * s24;
-  float u2 = (float)(2u * (r.z >> 9) + 1u) * s24;
-  float u3 = (float)(2u * (r.w >> 9) + 1u) * s24;
+  const float u0 = philox_uniform(r.x), u1 = philox_uniform(r.y), u2 = philox_uniform(r.z), u3 = philox_uniform(r.w);
   float ra = sqrtf(-2.0f * logf(u0));
   float rb = sqrtf(-2.0f * logf(u2));
   // the angle 2 pi u taken as 2 pi (u - 1/2) + pi, within [-pi, pi] where the
