@@ -37,6 +37,7 @@ constexpr int kMaxMx = 825, kMaxMy = 875, kMaxMz = 588;
 
 constexpr int kMaxZCand = 6;
 constexpr int kMaxPCand = 4;
+constexpr int kTuneReps = 3;  // timed launches per candidate and round
 
 struct WSrc;  // fsl_fft_reg.cuh
 
@@ -716,18 +717,18 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
     return;
   }
   // three rounds over the candidates in turn (clock ramp-up and cold caches
-  // hit every candidate alike), five launches each, the fastest round kept
+  // hit every candidate alike), kTuneReps launches each, the fastest round kept
   for (int i = 0; i < fp->nzc; ++i) fp->zc_us[i] = 1e30f;
   for (int round = 0; round < 3 && fp->nzc > 1; ++round)
     for (int i = 0; i < fp->nzc; ++i) {
       use_zcand(fp, i);
       zsolve(B, fp, s);  // warm-up
       cudaEventRecord(e0, s);
-      for (int r = 0; r < 5; ++r) zsolve(B, fp, s);
+      for (int r = 0; r < kTuneReps; ++r) zsolve(B, fp, s);
       cudaEventRecord(e1, s);
       float ms = 0.f;
       if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) ms = 1e9f;
-      fp->zc_us[i] = std::min(fp->zc_us[i], ms * 1000.f / 5.f);
+      fp->zc_us[i] = std::min(fp->zc_us[i], ms * 1000.f / kTuneReps);
     }
   int best = 0;
   for (int i = 1; i < fp->nzc; ++i)
@@ -747,11 +748,11 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
         use_pcand(fp, i);
         reg_transform(B, fp, s, none, ws);  // warm-up
         cudaEventRecord(e0, s);
-        for (int r = 0; r < 5; ++r) reg_transform(B, fp, s, none, ws);
+        for (int r = 0; r < kTuneReps; ++r) reg_transform(B, fp, s, none, ws);
         cudaEventRecord(e1, s);
         float ms = 0.f;
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) ms = 1e9f;
-        fp->pc_us[i] = std::min(fp->pc_us[i], ms * 1000.f / 5.f);
+        fp->pc_us[i] = std::min(fp->pc_us[i], ms * 1000.f / kTuneReps);
       }
     int pbest = 0;
     for (int i = 1; i < fp->npc; ++i)
@@ -767,11 +768,11 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
         fp->use_lines = sc == 1;
         reg_transform(B, fp, s, none);  // warm-up
         cudaEventRecord(e0, s);
-        for (int r = 0; r < 5; ++r) reg_transform(B, fp, s, none);
+        for (int r = 0; r < kTuneReps; ++r) reg_transform(B, fp, s, none);
         cudaEventRecord(e1, s);
         float ms = 0.f;
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) ms = 1e9f;
-        fp->sched_us[sc] = std::min(fp->sched_us[sc], ms * 1000.f / 5.f);
+        fp->sched_us[sc] = std::min(fp->sched_us[sc], ms * 1000.f / kTuneReps);
       }
     fp->use_lines = fp->sched_us[1] < fp->sched_us[0];
   }
