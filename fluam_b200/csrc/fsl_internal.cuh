@@ -516,7 +516,8 @@ __device__ __forceinline__ bool quad_of(int blk, int np, long& e, int& a, int& q
 // flight within a few planes of it.  Bonded instances keep the order in
 // memory: beads of a chain follow each other there, and their warps share
 // stencil nodes.  Which place takes a particle changes no sum (the list may
-// be many steps old: it only has to be a permutation).
+// be many steps old: it only has to be a permutation).  Only a step's
+// launches may call it: their first force evaluation has built the list.
 __device__ __forceinline__ int particle_at(const Rep& R, long e) {
   if (!R.P.order || R.P.bonded) return (int)e;
   const int i = R.sorted[e];

@@ -1467,9 +1467,11 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_spread(FSL_KARGS, int drift
   const bool cell_mode = own_forces ? vl_state(R, blk) : false;
   if (!quad_of(blk, np, e, a, qb)) return;
   const bool on = e < np;  // lanes past the end join the shuffles only
-  // cell order on the cell-list path (a list the step has just built)
+  // cell order where a step has built the lists (ordered): the list of this
+  // evaluation on the cell-list path, the last rebuild's on the Verlet path;
+  // fsl_spread may come before any list and takes memory order
   const bool by_cell = ordered && !P.verlet && !P.nolist;
-  const int i = on ? (by_cell ? cell_list(R, drift == 1).sorted[e] : particle_at(R, e)) : 0;
+  const int i = on ? (by_cell ? cell_list(R, drift == 1).sorted[e] : ordered ? particle_at(R, e) : (int)e) : 0;
   bool sat = false;
   QuadStencil<KN> S;
   {
