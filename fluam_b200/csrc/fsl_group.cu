@@ -1223,6 +1223,38 @@ void exec_enqueue(Exec& e) {
   if (e.io_out) e.io_out(e.stream);
 }
 
+// A launch of the groups' step was refused: the stage that it belongs to.
+int launch_refused(Group* const* groups, size_t n, cudaError_t err) {
+  for (size_t i = 0; i < n; ++i) {
+    const Group* g = groups[i];
+    if (g->fail_stage)
+      return errorf(FSL_E_CUDA, "kernel launch (stage %s, cells %d %d %d, kernel %d, %d instances): %s", g->fail_stage, g->key.mx,
+                    g->key.my, g->key.mz, g->key.kernel, g->B.nrep, cudaGetErrorString(err));
+  }
+  return cuda_fail(err, "kernel launch");
+}
+
+// Captures what `enqueue` puts on `s`.  A launch that is refused leaves a
+// graph without its node, which would replay the rest: such a graph is
+// dropped and the refusal returned.  (An error left by an earlier call of this
+// thread is none of the step's.)
+template <class F>
+int capture(cudaStream_t s, Group* const* groups, size_t n, F&& enqueue, cudaGraph_t* graph) {
+  cudaGetLastError();
+  FSL_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+  enqueue();
+  const cudaError_t le = cudaGetLastError();
+  cudaGraph_t g = nullptr;
+  const cudaError_t ce = cudaStreamEndCapture(s, &g);
+  if (le == cudaSuccess && ce == cudaSuccess) {
+    *graph = g;
+    return FSL_OK;
+  }
+  if (ce == cudaSuccess && g) cudaGraphDestroy(g);
+  cudaGetLastError();
+  return le != cudaSuccess ? launch_refused(groups, n, le) : cuda_fail(ce, "graph capture");
+}
+
 }  // namespace
 
 int exec_step(Exec& e, int64_t nsteps) {
@@ -1235,27 +1267,15 @@ int exec_step(Exec& e, int64_t nsteps) {
   for (int64_t k = 0; k < nsteps; ++k) {
     if (e.use_graph && e.steps > 0) {
       if (!e.gexec) {
-        FSL_TRY(cudaStreamBeginCapture(e.stream, cudaStreamCaptureModeThreadLocal));
-        exec_enqueue(e);
-        cudaGraph_t g = nullptr;
-        cudaError_t ce = cudaStreamEndCapture(e.stream, &g);
-        if (ce != cudaSuccess) return cuda_fail(ce, "graph capture");
-        e.graph = g;
-        FSL_TRY(cudaGraphInstantiate(&e.gexec, g, 0));
+        if ((rc = capture(e.stream, e.groups.data(), e.groups.size(), [&] { exec_enqueue(e); }, &e.graph))) return rc;
+        FSL_TRY(cudaGraphInstantiate(&e.gexec, e.graph, 0));
         e.captures++;
       }
       FSL_TRY(cudaGraphLaunch(e.gexec, e.stream));
     } else {
       exec_enqueue(e);
-      cudaError_t le = cudaGetLastError();
-      if (le != cudaSuccess) {
-        for (Group* g : e.groups)
-          if (g->fail_stage)
-            return errorf(FSL_E_CUDA, "kernel launch (stage %s, cells %d %d %d, kernel %d, %d instances): %s",
-                          g->fail_stage, g->key.mx, g->key.my, g->key.mz, g->key.kernel, g->B.nrep,
-                          cudaGetErrorString(le));
-        return cuda_fail(le, "kernel launch");
-      }
+      const cudaError_t le = cudaGetLastError();
+      if (le != cudaSuccess) return launch_refused(e.groups.data(), e.groups.size(), le);
     }
     e.steps++;
     for (Group* g : e.groups) {
@@ -1290,12 +1310,9 @@ int exec_step_each(Exec& e, int64_t nsteps) {
     group_shape(g, shape);
     if (!g.gexec || shape != g.shape) {
       group_drop_graph(g);
-      g.shape = shape;
-      FSL_TRY(cudaStreamBeginCapture(g.stream, cudaStreamCaptureModeThreadLocal));
-      group_enqueue_step(g);
-      const cudaError_t ce = cudaStreamEndCapture(g.stream, &g.graph);
-      if (ce != cudaSuccess) return cuda_fail(ce, "graph capture");
+      if (int rc = capture(g.stream, &e.groups[i], 1, [&] { group_enqueue_step(g); }, &g.graph)) return rc;
       FSL_TRY(cudaGraphInstantiate(&g.gexec, g.graph, 0));
+      g.shape = shape;
       e.captures++;
     }
     total += g.launches;
