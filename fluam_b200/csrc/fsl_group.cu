@@ -1136,6 +1136,10 @@ void group_shape(const Group& g, std::vector<long long>& shape) {
   shape.push_back(g.prof.on ? 1 : 0);
   shape.push_back((long long)(uintptr_t)g.io_in);
   shape.push_back((long long)(uintptr_t)g.io_out);
+  // by copies, or by kernels through the buffers' device addresses
+  shape.push_back(g.io_kernels ? 1 : 0);
+  shape.push_back((long long)(uintptr_t)(g.io_kernels ? g.io_in_dev : nullptr));
+  shape.push_back((long long)(uintptr_t)(g.io_kernels ? g.io_out_dev : nullptr));
   // the pair path of the instances and the list build launch other kernels
   shape.push_back(g.B.has_vl | g.B.has_cl << 1 | (g.B.lists_pick + 1) << 2);
   for (int k = 0; k < NKIND; ++k) shape.push_back(g.B.nblk[k]);

@@ -116,10 +116,40 @@ static int refused(bool each) {
   return 0;
 }
 
+// An input/output step by kernels holds the buffers' device addresses: the
+// same host addresses with other ones, or with copies, need a new graph.
+static int io_key() {
+  One a;
+  CHECK(a.make(8, 3) == 0);
+  Exec e;
+  CHECK(exec_init(e, 0) == 0);
+  e.groups = {&a.g};
+  std::vector<double> host(9), map1(9), map2(9);
+  auto step = [&](double* in, double* out, bool kernels) {
+    a.g.io_in = a.g.io_out = host.data();
+    a.g.io_bytes = sizeof(double) * 9;
+    a.g.io_kernels = kernels;
+    a.g.io_in_dev = in;
+    a.g.io_out_dev = out;
+    return exec_step(e, 1);
+  };
+  CHECK(exec_step(e, 1) == FSL_OK);
+  const auto c0 = e.captures;
+  CHECK(step(map1.data(), map1.data(), true) == FSL_OK && e.captures == c0 + 1);
+  CHECK(step(map1.data(), map1.data(), true) == FSL_OK && e.captures == c0 + 1);
+  CHECK(step(map2.data(), map1.data(), true) == FSL_OK && e.captures == c0 + 2);
+  CHECK(step(map2.data(), map2.data(), true) == FSL_OK && e.captures == c0 + 3);
+  CHECK(step(nullptr, nullptr, false) == FSL_OK && e.captures == c0 + 4);
+  e.groups.clear();
+  exec_destroy(e);
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "refused") return refused(false);
   if (what == "refused_each") return refused(true);
+  if (what == "io_key") return io_key();
   std::printf("unknown test\n");
   return 2;
 }
