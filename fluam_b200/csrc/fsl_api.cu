@@ -209,8 +209,7 @@ int fsl_set_positions(fsl_handle* h, const double* in) {
 int fsl_step_io(fsl_handle* h, const double* in, double* out) {
   if (!h || !in || !out) return errorf(FSL_E_ARG, "null argument");
   FSL_TRY(cudaSetDevice(h->exec.device));
-  void *din = nullptr, *dout = nullptr;
-  if (!fsl::pinned_host(in, &din) || !fsl::pinned_host(out, &dout)) {
+  if (!fsl::pinned_host(in) || !fsl::pinned_host(out)) {
     // pageable buffers: the copies stay outside the step's graph
     if (int rc = fsl_set_positions(h, in)) return rc;
     if (int rc = fsl_step(h, 1)) return rc;
@@ -220,9 +219,11 @@ int fsl_step_io(fsl_handle* h, const double* in, double* out) {
   g.io_in = in;
   g.io_out = out;
   g.io_bytes = sizeof(double) * 3 * (size_t)params(h).np;
-  g.io_kernels = din && dout && params(h).np <= fsl::kIoKernelNp;
-  g.io_in_dev = (const double*)din;
-  g.io_out_dev = (double*)dout;
+  const size_t n3 = 3 * (size_t)params(h).np;
+  const bool small = params(h).np <= fsl::kIoKernelNp;
+  g.io_in_dev = small ? fsl::mapped_doubles(in, n3) : nullptr;
+  g.io_out_dev = small ? fsl::mapped_doubles(out, n3) : nullptr;
+  g.io_kernels = g.io_in_dev && g.io_out_dev;
   const int rc = fsl::exec_step(h->exec, 1);
   g.io_in = nullptr;
   g.io_out = nullptr;

@@ -1,5 +1,7 @@
 // fsl_group.cu -- slots, size-class groups and the graph-captured step of
 // any number of groups (declared in fsl_group.cuh).
+#include <cuda.h>
+
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -1075,14 +1077,46 @@ void exec_drop_graph(Exec& e) {
   e.shape.clear();
 }
 
-bool pinned_host(const void* p, void** dev) {
+bool pinned_host(const void* p) {
   cudaPointerAttributes a{};
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  if (dev) *dev = a.devicePointer;
   return a.type == cudaMemoryTypeHost;
+}
+
+namespace {
+using PointerGetAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+
+PointerGetAttributes pointer_get_attributes() {
+  static const PointerGetAttributes f = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult st = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &p, 12000, cudaEnableDefault, &st) != cudaSuccess ||
+        st != cudaDriverEntryPointSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    return (PointerGetAttributes)p;
+  }();
+  return f;
+}
+}  // namespace
+
+double* mapped_doubles(const void* p, size_t n) {
+  const PointerGetAttributes get = pointer_get_attributes();
+  if (!get || !n || (uintptr_t)p % alignof(double)) return nullptr;
+  CUdeviceptr dev = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute a[3] = {CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                              CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* out[3] = {&dev, &start, &size};
+  if (get(3, a, out, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS || !dev) return nullptr;
+  // the range in host addresses, as p is
+  const uintptr_t at = (uintptr_t)p - (uintptr_t)start;
+  if ((uintptr_t)p < (uintptr_t)start || at > size || size - at < n * sizeof(double)) return nullptr;
+  return (double*)(uintptr_t)dev;
 }
 
 void exec_destroy(Exec& e) {

@@ -173,8 +173,13 @@ struct Exec {
 };
 
 // Whether p is page-locked host memory (a copy from or to it can be a node
-// of a CUDA graph); dev: its address on the device (null: not mapped).
-bool pinned_host(const void* p, void** dev = nullptr);
+// of a CUDA graph).
+bool pinned_host(const void* p);
+// The device address of n doubles at p if kernels can read and write them
+// there: page-locked in one piece and aligned (a copy takes any address, and
+// the driver refuses one past the end of a registration; a kernel would
+// fault).  Null otherwise.
+double* mapped_doubles(const void* p, size_t n);
 
 int exec_init(Exec& e, int device);
 void exec_destroy(Exec& e);

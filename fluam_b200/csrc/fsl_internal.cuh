@@ -747,7 +747,10 @@ void launch_reset_lists(const Rep& r, cudaStream_t s);
 void launch_moved_check(const Rep& r, cudaStream_t s);
 // The ends of an input/output step of at most kIoKernelNp particles: q from
 // the device address `in` of page-locked host memory with the check of
-// launch_moved_check; q to `out` with the step counter.
+// launch_moved_check; q to `out` with the step counter.  A step by kernels
+// and by copy nodes: 16^3, 16 particles 50.5 and 55.1 us; 64^3, 4,096 103.5
+// and 106.8; 128^3, 16,384 324.8 and 329.9, 32,768 330.3 and 328.9, 65,536
+// 371.1 and 367.0 (64^3 still gains there, 203.6 and 207.3).
 constexpr int kIoKernelNp = 16384;
 void launch_io_in(const Rep& r, const double* in, cudaStream_t s);
 void launch_io_out(const Rep& r, double* out, cudaStream_t s);

@@ -1,5 +1,6 @@
 // A CUDA runtime without a device: device memory is host memory, streams and
 // events are handles, graph launches are counted.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -7,6 +8,20 @@
 
 cudaError_t g_last = cudaSuccess;
 int g_launched = 0;
+// the one page-locked range and its place on the device
+char *g_pin = nullptr, *g_pin_dev = nullptr;
+size_t g_pin_bytes = 0;
+
+static CUresult pointer_attributes(unsigned n, CUpointer_attribute* a, void** out, CUdeviceptr p) {
+  char* c = (char*)p;
+  const bool in = c >= g_pin && c < g_pin + g_pin_bytes;
+  for (unsigned i = 0; i < n; ++i)
+    if (a[i] == CU_POINTER_ATTRIBUTE_DEVICE_POINTER) *(CUdeviceptr*)out[i] = in ? (CUdeviceptr)(g_pin_dev + (c - g_pin)) : 0;
+    else if (a[i] == CU_POINTER_ATTRIBUTE_RANGE_START_ADDR) *(CUdeviceptr*)out[i] = in ? (CUdeviceptr)g_pin : 0;
+    else if (a[i] == CU_POINTER_ATTRIBUTE_RANGE_SIZE) *(size_t*)out[i] = in ? g_pin_bytes : 0;
+    else return CUDA_ERROR_INVALID_VALUE;
+  return CUDA_SUCCESS;
+}
 
 extern "C" {
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
@@ -42,4 +57,10 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) { free((void*)s); return cudaSucce
 cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus* s) { *s = cudaStreamCaptureStatusActive; return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaGetDriverEntryPointByVersion(const char* name, void** f, unsigned, unsigned long long, cudaDriverEntryPointQueryResult* st) {
+  const bool known = !std::strcmp(name, "cuPointerGetAttributes");
+  *f = known ? (void*)pointer_attributes : nullptr;
+  *st = known ? cudaDriverEntryPointSuccess : cudaDriverEntryPointSymbolNotFound;
+  return cudaSuccess;
+}
 }

@@ -11,6 +11,8 @@
 
 extern cudaError_t g_last;  // the runtime's last error (counting_cudart.cpp)
 extern int g_launched;      // graphs launched
+extern char *g_pin, *g_pin_dev;  // the one page-locked range
+extern size_t g_pin_bytes;
 static int g_refuse = 0;    // the next launches of the noise that are refused
 
 #define CHECK(c)                                                 \
@@ -145,11 +147,32 @@ static int io_key() {
   return 0;
 }
 
+// Kernels may take a buffer that lies in the page-locked range as a whole
+// and is aligned; everything else is left to copies.
+static int mapped() {
+  std::vector<double> mem(100), dev(100);
+  g_pin = (char*)(mem.data() + 10);
+  g_pin_dev = (char*)dev.data();
+  g_pin_bytes = 50 * sizeof(double);
+  for (size_t n : {1, 6, 48, 50})
+    for (size_t at : {0, 2, 44, 49}) {
+      double* got = mapped_doubles(mem.data() + 10 + at, n);
+      CHECK(got == (at + n <= 50 ? dev.data() + at : nullptr));
+    }
+  CHECK(!mapped_doubles(mem.data() + 9, 1) && !mapped_doubles(mem.data() + 60, 1));
+  CHECK(!mapped_doubles((char*)(mem.data() + 10) + 4, 6));
+  CHECK(!mapped_doubles(mem.data() + 10, 0));
+  g_pin_bytes -= 4;  // the last double is cut
+  CHECK(mapped_doubles(mem.data() + 10, 49) && !mapped_doubles(mem.data() + 10, 50));
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "refused") return refused(false);
   if (what == "refused_each") return refused(true);
   if (what == "io_key") return io_key();
+  if (what == "mapped") return mapped();
   std::printf("unknown test\n");
   return 2;
 }

@@ -24,7 +24,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("what", ["refused", "refused_each", "io_key"])
+@pytest.mark.parametrize("what", ["refused", "refused_each", "io_key", "mapped"])
 def test_step_host(program, what):
     r = subprocess.run([program, what], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -85,6 +85,26 @@ def test_step_io_then_plain_steps(fsl):
     b.close()
 
 
+def test_step_io_unaligned_buffer(fsl):
+    """Page-locked doubles at an address that is no multiple of 8 (or of 4):
+    taken by copies, which have no alignment."""
+    import torch
+    cfg = _config(fsl)
+    q0 = uniform_positions(100, (48, 48, 48), 9)
+    a, b = fsl.StokesLimit(cfg, q0), fsl.StokesLimit(cfg, q0)
+    raw = torch.empty(q0.nbytes + 8, dtype=torch.uint8).pin_memory()
+    for off in (4, 1, 0):
+        view = raw.numpy()[off:off + q0.nbytes]
+        view[:] = np.frombuffer(q0.tobytes(), np.uint8)
+        a.step_io(raw.data_ptr() + off, raw.data_ptr() + off)
+        b.set_positions(q0)
+        b.step(1)
+        q0 = b.positions()
+        np.testing.assert_array_equal(np.frombuffer(view.tobytes()).reshape(q0.shape), q0)
+    a.close()
+    b.close()
+
+
 @pytest.mark.parametrize("pinned", [True, False], ids=["pinned", "pageable"])
 def test_batch_step_io_equals_set_step_get(fsl, pinned):
     """The batched form: every instance of a batch over three size classes
