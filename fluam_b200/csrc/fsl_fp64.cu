@@ -274,16 +274,26 @@ __global__ void __launch_bounds__(kPartThreads) k_interp_update64(FSL_KARGS, int
   for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
     for (int d = 0; d < 3; ++d) us[d] += __shfl_xor_sync(0xffffffffu, us[d], o);
-  if (lane >= 3) return;
-  const size_t k = (size_t)lane * np + i;
+  const int comp = lane < 3 ? lane : 0;  // the other lanes join the shuffles
+  const size_t k = (size_t)comp * np + i;
   const double h = stage == 1 ? 0.5 * P.dt : P.dt;
-  double r = R.q[k] + h * (lane == 0 ? us[0] : (lane == 1 ? us[1] : us[2]));
+  double r = R.q[k] + h * (comp == 0 ? us[0] : (comp == 1 ? us[1] : us[2]));
   if (P.has_extra) {
-    const size_t nb = (size_t)6 * P.nc + (size_t)(3 + lane) * np + i;
+    const size_t nb = (size_t)6 * P.nc + (size_t)(3 + comp) * np + i;
     double xi = R.noise64[nb];
     if (stage == 2) xi += R.noise64[nb + (size_t)3 * np];
     r += h * P.extra_mob * R.F[k] + P.fact2 * xi;
   }
+  if (P.verlet) {
+    // a particle beyond half the skin from its reference position: the list
+    // is rebuilt at the next evaluation (k_interp_update)
+    const double d = lane < 3 ? r - R.qref[k] : 0.0;
+    double d2 = d * d;
+    d2 += __shfl_xor_sync(0xffffffffu, d2, 1);
+    d2 += __shfl_xor_sync(0xffffffffu, d2, 2);
+    if (lane == 0 && d2 > P.vl_half2) R.vl_flag[stage == 1 ? 1 : 0] = *R.t + stage;
+  }
+  if (lane >= 3) return;
   if (!isfinite(r)) set_err(R.err, 2);
   qout[k] = r;
 }

@@ -56,6 +56,35 @@ def test_verlet_follows_cell_list(fsl, scheme):
         assert a.status()["error_bits"] == 0 and b.status()["error_bits"] == 0
 
 
+@pytest.mark.parametrize("pair", ["PAIR_SOFT", "PAIR_TABLE_LJ"])
+@pytest.mark.parametrize("scheme", [0, 1])
+def test_fp64_form_follows_cell_list(fsl, monkeypatch, scheme, pair):
+    """The FP64 form with particles that leave the skin: its update asks for
+    the rebuilds as the other forms' do."""
+    soft = pair == "PAIR_SOFT"
+    m = 24
+    per = m // (2 if soft else 3)
+    g = (np.stack(np.meshgrid(*[np.arange(per)] * 3)).reshape(3, -1) + 0.5) * (m / per) - m / 2
+    q = g + np.random.default_rng(11).uniform(-0.3, 0.3, g.shape)
+    cfg = fsl.make_config((m,) * 3, (float(m),) * 3, eta=1.0, kT=0.5, dt=0.03, cutoff=1.5 if soft else 3.0, kernel=3,
+                          pair=getattr(fsl, pair), soft_epsilon=5.0, seed=9, scheme=scheme, precision=2)
+    monkeypatch.setenv("FLUAMSL_VERLET", "0")
+    a = fsl.StokesLimit(cfg, q)
+    monkeypatch.setenv("FLUAMSL_VERLET", "1")
+    b = fsl.StokesLimit(cfg, q)
+    with a, b:
+        for _ in range(3):
+            a.step(10)
+            b.step(10)
+            qa, qb = a.positions(), b.positions()
+            span = np.abs(qa - q).max()
+            assert span > 0.35  # past skin / 2
+            # rounding alone for the soft force; the table's 8-bit filter
+            # turns it into single steps of 2e-6 of a force
+            assert np.abs(qa - qb).max() <= (1e-9 if soft else 1e-4) * span
+        assert a.status()["error_bits"] == 0 and b.status()["error_bits"] == 0
+
+
 def test_verlet_after_set_positions_and_entry_points(fsl):
     q = uniform_positions(400, (32.0,) * 3, 3)
     a, b = _pair(fsl, q, kT=0.01, dt=0.01)
