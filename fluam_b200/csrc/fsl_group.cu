@@ -96,7 +96,7 @@ SlotLayout layout(const Params& P, int np_cap) {
   L.vl_cnt = take(two_lists ? sizeof(int) * np : 0);
   L.vl_idx = take(two_lists ? sizeof(int) * (size_t)kVlCap * np : 0);
   L.qref = take(two_lists ? sizeof(double) * 3 * np : 0);
-  L.vl_flag = take(sizeof(uint64_t) * 3);
+  L.vl_flag = take(sizeof(uint64_t) * kVlWords);
   L.bar = take(sizeof(unsigned) * 2);
   L.total = off;
   return L;
@@ -253,11 +253,13 @@ int make_params(const fsl_config& c, int64_t np, Params& P) {
   // within two cells), no list at all without pair forces.  The table of the
   // Lennard-Jones force is exactly zero from rc on, so pairs beyond rc on the
   // list add nothing; its cutoffs are several particles wide, so its skin is
-  // smaller, and a density that would fill the kVlCap slots (40 expected
-  // neighbours of 64, five standard deviations of a uniform density) keeps
-  // it on the cell-list kernel.  At 64^3 cells, 8,000 particles, rc = 5 the
+  // smaller, and a density that would often fill the kVlCap slots keeps it on
+  // the cell-list kernel: beyond 40 expected neighbours, 24 of which (3.8
+  // standard deviations of a uniform density) are left to chance.  A list
+  // that overflows all the same, or that particles outrun, gives way to the
+  // cell list (vl_no_build).  At 64^3 cells, 8,000 particles, rc = 5 the
   // cell list, rebuilt for each evaluation, and its force kernel took 83 of
-  // 238 us of a step's kernels; from the list a step is 147 us instead of 210.
+  // 238 us of a step's kernels.
   // FLUAMSL_VERLET=0 keeps pair forces on the cell-list kernel.
   if (c.scheme <= FSL_SCHEME_FIRST_ORDER && np > 0) {
     const bool pairs_on = c.nonbonded && c.pair != FSL_PAIR_NONE;
@@ -272,6 +274,8 @@ int make_params(const fsl_config& c, int64_t np, Params& P) {
       P.skin = skin;
       P.vl_cut2 = (c.cutoff + skin) * (c.cutoff + skin);
       P.vl_half2 = 0.25 * skin * skin;
+      // a build takes longer the more neighbours there are
+      P.vl_soon = std::max(1, (int)(0.6 * expect));
       P.order = 24.0 * P.nc > kOrderBytes;
     }
   }
@@ -438,7 +442,7 @@ int slot_clear_errors(Slot& s, cudaStream_t st) {
 }
 
 int slot_force_lists(Slot& s, cudaStream_t st) {
-  static const uint64_t flags[3] = {0, 0, 1};
+  static const uint64_t flags[kVlWords] = {0, 0, 1};
   FSL_TRY(cudaMemcpyAsync(s.r.vl_flag, flags, sizeof(flags), cudaMemcpyHostToDevice, st));
   return FSL_OK;
 }
@@ -680,8 +684,9 @@ int group_upload(Group& g) {
     B.max_np = std::max(B.max_np, s->np_cap);
     B.max_noise_n = std::max<uint64_t>(B.max_noise_n, noise_count(g.P0, s->np_cap));
     B.tiled = B.tiled && tile_eligible(s->r.P);  // per instance: the cell sizes
-    if (s->r.P.verlet || s->r.P.nolist) B.has_vl = 1;
-    else B.has_cl = 1;
+    const Params& P = s->r.P;
+    if (P.verlet || P.nolist) B.has_vl = 1;
+    if (!(P.verlet || P.nolist) || (P.verlet && P.pair == FSL_PAIR_TABLE_LJ)) B.has_cl = 1;
   }
   if (n > g.d_cap) {
     if (g.d_reps || g.d_boff) {

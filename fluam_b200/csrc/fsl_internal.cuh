@@ -58,6 +58,7 @@ struct Params {
   // rc + skin at the reference positions qref, rebuilt when a particle has
   // moved more than skin / 2 since; nolist: no pair forces, no cell list
   int verlet, nolist;
+  int vl_soon;  // Lennard-Jones: evaluations between two list builds below which the list does not pay (vl_no_build)
   int order;  // spread and interpolation take the particles in cell order (particle_at)
   double skin, vl_cut2, vl_half2;  // skin, (rc + skin)^2, (skin / 2)^2
   int has_extra;
@@ -460,8 +461,12 @@ struct Rep {
   // (counter + 1) at whose force evaluation at q (0) or q^{n+1/2} (1) the
   // list must be rebuilt; [2] 1: rebuild at the next evaluation, 2: cell
   // list requested by an entry point, 3: cell mode (a particle had more
-  // than kVlCap neighbours: the pair forces come from the cell list of every
-  // evaluation until the positions are set again)
+  // than kVlCap neighbours, or Lennard-Jones particles outran the list: the
+  // pair forces come from the cell list of every evaluation, for the soft
+  // force until the instance's lists are reset or an entry point builds them,
+  // for the table kVlCellSteps steps at least, lj_cells); [3] the force
+  // evaluation of the last list build (vl_now); [4] the step counter when
+  // cell mode began
   int* vl_cnt;
   int* vl_idx;
   double* qref;
@@ -471,6 +476,7 @@ struct Rep {
 };
 constexpr int kCoopMaxBlocks = 1024;
 constexpr int kVlCap = 64;
+constexpr int kVlWords = 5;
 constexpr int kObsVals = 10;      // msd, displacement[3], force[3], momentum[3]
 constexpr int kObsSlots = 16;     // steps, msd, msd_sum, disp[3], force[3], mom[3], mom_sum[3]
 constexpr int kObsMaxBlocks = 148;
@@ -496,6 +502,49 @@ __device__ __forceinline__ bool list_needed(const Rep& R, int which) {
   if (R.P.nolist) return false;
   // 3: cell mode (the list overflowed): a cell list at every evaluation
   return f != 0 || R.vl_flag[which] == *R.t + 1;
+}
+
+// A list build of the Lennard-Jones table's long cutoff costs many
+// evaluations' worth of what the list saves (one thread a particle through
+// up to 125 cells: 64^3 with 9,261 particles of 26 neighbours 650 us, where
+// the step is 111 us with the list kept and 173 from the cell list; 32^3 with
+// 1,000 particles of 23 neighbours 250, 74 and 137 us; 1,000 of 3 neighbours
+// in 64^3 20, 83 and 128 us).  So a movement rebuild that comes P.vl_soon
+// evaluations (two a step) or less after the last build puts such an instance
+// into cell mode, whose forces are k_forces', and after kVlCellSteps steps
+// the list is tried again; a list that overflows does the same.  9,261
+// particles that cross the skin at every evaluation: 1417 us a step with a
+// build each time, 188 so.  Both decisions follow from the instance's own
+// words, alone and in a batch alike.
+constexpr int kVlCellSteps = 256;
+
+// The number of force evaluation `which` of the step at hand (from 1).
+__device__ __forceinline__ uint64_t vl_now(const Rep& R, int which) { return 2 * *R.t + which + 1; }
+
+// Whether the pair forces of a Lennard-Jones instance with a Verlet list come
+// from the cell list now (k_forces).
+__device__ __forceinline__ bool lj_cells(const Rep& R) { return R.P.verlet && R.P.pair == 1 && R.vl_flag[2] == 3; }
+
+// Before a list build, by every thread that would take part in it: true if
+// there is to be none.  (Who reads the word of the last build after another
+// thread of this build has set it finds the present evaluation there.)
+__device__ __forceinline__ bool vl_no_build(const Rep& R, int which) {
+  const uint64_t f = R.vl_flag[2];
+  if (f == 3) return true;
+  if (f != 0 || R.P.pair != 1) return false;
+  const uint64_t now = vl_now(R, which), last = R.vl_flag[3];
+  if (last == 0 || last == now || now - last > (uint64_t)R.P.vl_soon) return false;
+  R.vl_flag[2] = 3;
+  R.vl_flag[4] = *R.t;
+  return true;
+}
+
+// The end of a step, by one thread: its counter, and the list of a
+// Lennard-Jones instance tried again.
+__device__ __forceinline__ void step_done(const Rep& R) {
+  const uint64_t t = *R.t + 1;
+  *R.t = t;
+  if (lj_cells(R) && t - R.vl_flag[4] >= kVlCellSteps) R.vl_flag[2] = 1;
 }
 
 // The quad of this thread in a KIND_T4 launch: particle index e (in the
@@ -554,7 +603,7 @@ struct Batch {
   int max_np;
   uint64_t max_noise_n;
   int tiled;        // spread and W build by launch_spread_w
-  int has_vl, has_cl;  // instances on the Verlet path / on the cell-list pair path
+  int has_vl, has_cl;  // instances on the Verlet path / that k_forces may serve (cell-list path, lj_cells)
   int nblk[NKIND];  // total blocks of each particle launch kind
   const Rep* one;   // host copy of the single instance (nrep == 1), else null
   // list build of a batch of small instances, as the class's tuner picked it

@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_forces(FSL_KARGS, int which
   if ((ig & ~3) >= P.np) return;  // uniform per warp (4 particles per warp)
   const bool active = ig < P.np;  // inactive lanes still join the shuffles
   const int np = P.np;
-  if (P.verlet || P.nolist) return;  // k_forces_vl
+  if (P.nolist || (P.verlet && !lj_cells(R))) return;  // k_forces_vl, k_spread
   // first-order scheme: forces at q^{n+1/2} only with extraMobility
   // (src/boundaryParticlesFunctionStokesLimitFirstOrder.cu:170-180)
   if (which == 1 && P.scheme == 1 && !P.has_extra) return;
@@ -536,14 +536,18 @@ __device__ void vl_build_one(const Rep& R, int i, int which) {
   R.qref[i] = xi;
   R.qref[np + i] = yi;
   R.qref[2 * np + i] = zi;
-  if (over) R.vl_flag[2] = 3;  // cell mode from now on
+  if (i == 0) R.vl_flag[3] = vl_now(R, which);
+  if (over) {  // cell mode from now on
+    R.vl_flag[2] = 3;
+    R.vl_flag[4] = *R.t;
+  }
 }
 
 template <bool ONE>
 __global__ void k_vl_build(FSL_KARGS, int which) {
   FSL_REP_FLAT(KIND_T1);
   const int i = blk * blockDim.x + threadIdx.x;
-  if (i >= P.np || !P.verlet || !list_needed(R, which) || R.vl_flag[2] == 3) return;
+  if (i >= P.np || !P.verlet || !list_needed(R, which) || vl_no_build(R, which)) return;
   vl_build_one(R, i, which);
 }
 
@@ -590,7 +594,7 @@ __global__ void k_io_out(const __grid_constant__ Rep R, double* __restrict__ out
   fsl_pdl_enter();
   const long n3 = 3l * R.P.np;
   for (long k = blockIdx.x * (long)blockDim.x + threadIdx.x; k < n3; k += (long)gridDim.x * blockDim.x) out[k] = R.q[k];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *R.t += 1;
+  if (blockIdx.x == 0 && threadIdx.x == 0) step_done(R);
 }
 
 void launch_io_in(const Rep& r, const double* in, cudaStream_t s) {
@@ -709,7 +713,7 @@ __global__ void __launch_bounds__(kCoopThreads) k_lists_coop(const __grid_consta
   for (int i = tid; i < np; i += nth) cell_rank_one(R, i, which);
   if (!P.verlet) return;
   if (!grid_barrier(R, spin_limit)) return;
-  if (R.vl_flag[2] == 3) return;  // cell mode: no pair list
+  if (vl_no_build(R, which)) return;
   for (int i = tid; i < np; i += nth) vl_build_one(R, i, which);
 }
 
@@ -764,7 +768,7 @@ __global__ void __launch_bounds__(kScanThreads) k_lists_block(FSL_KARGS, int whi
   for (int i = threadIdx.x; i < np; i += blockDim.x) cell_rank_one(R, i, which);
   if (!P.verlet) return;
   __syncthreads();
-  if (R.vl_flag[2] == 3) return;  // cell mode: no pair list
+  if (vl_no_build(R, which)) return;
   for (int i = threadIdx.x; i < np; i += blockDim.x) vl_build_one(R, i, which);
 }
 
@@ -860,7 +864,7 @@ __device__ __forceinline__ void quad_force_vl(const Params& P, const Rep& R, int
   if (P.bonded && on) quad_bonds(R, q, np, i, a, rx, ry, rz, fx, fy, fz);
   if (P.verlet && on && cell_mode) {
     // the 27 neighbour cells of the current cell list, lanes taking cells
-    // a, a + 4, ...
+    // a, a + 4, ... (the table's cell mode is k_forces)
     const CellList cl = cell_list(R, which);
     const int cx = cellidx(minimage(rx, P.invlx, P.lx), P.invdnx, P.mnx),
               cy = cellidx(minimage(ry, P.invly, P.ly), P.invdny, P.mny),
@@ -984,6 +988,7 @@ __global__ void k_forces_vl(FSL_KARGS, int which) {
   const int np = P.np;
   if (!(P.verlet || P.nolist)) return;
   const bool cell_mode = vl_state(R, blk);
+  if (cell_mode && P.pair == 1) return;  // k_forces
   if (!quad_of(blk, np, e, a, qb)) return;
   // first-order scheme: forces at q^{n+1/2} only with extraMobility
   // (src/boundaryParticlesFunctionStokesLimitFirstOrder.cu:170-180)
@@ -1463,8 +1468,9 @@ __global__ void __launch_bounds__(kPartThreads, 4) k_spread(FSL_KARGS, int drift
   const int np = P.np;
   // forces: the Verlet-list and bonded forces at the spread's positions are
   // computed here (k_forces_vl's arithmetic) and stored, instead of read
-  const bool own_forces = forces && (P.verlet || P.nolist);
-  const bool cell_mode = own_forces ? vl_state(R, blk) : false;
+  const bool listed = forces && (P.verlet || P.nolist);
+  const bool cell_mode = listed ? vl_state(R, blk) : false;
+  const bool own_forces = listed && !(cell_mode && P.pair == 1);  // (then k_forces has left them in F)
   if (!quad_of(blk, np, e, a, qb)) return;
   const bool on = e < np;  // lanes past the end join the shuffles only
   // cell order where a step has built the lists (ordered): the list of this
@@ -1614,8 +1620,9 @@ template <bool ONE, int KN>
 __global__ void __launch_bounds__(kPartThreads) k_spread_wide(FSL_KARGS, int drift, int ordered, int forces, int cache) {
   FSL_REP_FLAT(KIND_T32);
   const int np = P.np;
-  const bool own_forces = forces && (P.verlet || P.nolist);
-  const bool cell_mode = own_forces ? vl_state(R, blk) : false;
+  const bool listed = forces && (P.verlet || P.nolist);
+  const bool cell_mode = listed ? vl_state(R, blk) : false;
+  const bool own_forces = listed && !(cell_mode && P.pair == 1);  // (then k_forces has left them in F)
   const int lane = threadIdx.x & 31;
   const long e = (blk * (long)blockDim.x + threadIdx.x) >> 5;
   if (e >= np) return;  // a whole warp
@@ -2231,7 +2238,7 @@ template <bool ONE>
 __global__ void k_step_counter(FSL_KARGS) {
   FSL_REP_AT(blockIdx.y);
   (void)P;
-  if (threadIdx.x == 0) *R.t += 1;
+  if (threadIdx.x == 0) step_done(R);
 }
 
 void launch_step_counter(const Batch& B, cudaStream_t s) {

@@ -4,6 +4,7 @@ FP64 oracle: forces of the same pairs to FP64 rounding, except where that
 rounding moves a pair by one step of the table's 8-bit filter; and steps with
 rebuilds, host position changes and a list that overflows."""
 import os
+import time
 
 import numpy as np
 import pytest
@@ -93,3 +94,66 @@ def test_overflow(fsl):
     assert rel_inf(a.positions() - q, b.positions() - q) < 1e-5
     a.close()
     b.close()
+
+
+def test_fast_particles_take_the_cells(fsl):
+    """Particles that outrun the list at every evaluation: the forces come
+    from the cell list, at its speed and with its values."""
+    m, q = 64, lattice(9261, 64, 9)
+    a, b = make(fsl, m, q, kT=1.0, dt=0.1), make(fsl, m, q, verlet="0", kT=1.0, dt=0.1)
+    us = []
+    for x in (a, b):
+        x.step(20)
+        x.sync()
+        t = []
+        for _ in range(3):
+            t0 = time.perf_counter()
+            x.step(40)
+            x.sync()
+            t.append(time.perf_counter() - t0)
+        us.append(min(t) / 40 * 1e6)
+    # a build at every evaluation took eight times the cell list's step
+    assert us[0] < 1.5 * us[1], us
+    for _ in range(3):
+        q = a.positions()
+        b.set_positions(q)
+        b.set_step(a.status()["step"])
+        for x in (a, b):
+            x.step(1)
+            x.sync()
+        assert rel_inf(a.positions() - q, b.positions() - q) < 1e-5
+    a.close()
+    b.close()
+
+
+def test_list_tried_again(fsl):
+    """Past the steps after which the list is tried again: an instance alone
+    and in a batch beside slow and soft ones, bit for bit, and the values of
+    the cell list on the way."""
+    m = 24
+    args = dict(eta=1.0, cutoff=5.0, kernel=3, seed=4)
+    cfg = [fsl.make_config((m,) * 3, (24.0,) * 3, kT=kT, dt=dt, pair=p, **args)
+           for kT, dt, p in [(0.5, 0.05, fsl.PAIR_TABLE_LJ), (0.01, 0.01, fsl.PAIR_TABLE_LJ), (0.5, 0.05, fsl.PAIR_SOFT)]]
+    qs = [lattice(400, m, 20 + i) for i in range(3)]
+    batch = fsl.Batch(cfg, qs)
+    alone = [fsl.StokesLimit(c, q) for c, q in zip(cfg, qs)]
+    b = make(fsl, m, qs[0], verlet="0", kT=0.5, dt=0.05)
+    for n in (5, 251, 1, 1, 1, 6, 255, 30):
+        batch.step(n)
+        batch.sync()
+        for i, a in enumerate(alone):
+            a.step(n)
+            a.sync()
+            np.testing.assert_array_equal(batch.positions(i), a.positions(), err_msg=f"{n} {i}")
+        # the fast instance's next step against the cell list's
+        q = alone[0].positions()
+        b.set_positions(q)
+        b.set_step(alone[0].status()["step"])
+        for x in (alone[0], b, batch):
+            x.step(1)
+            x.sync()
+        for a in alone[1:]:
+            a.step(1)
+        assert rel_inf(alone[0].positions() - q, b.positions() - q) < 1e-5, n
+    for x in alone + [b, batch]:
+        x.close()
