@@ -91,11 +91,11 @@ SlotLayout layout(const Params& P, int np_cap) {
   L.start1 = take(two_lists ? sizeof(int) * (mN + 1) : 0);
   L.sorted1 = take(two_lists ? sizeof(int) * np : 0);
   L.ws1 = take(two_lists ? sizeof(double) * 3 * np : 0);
-  // for every pair potential: a slot of a server's class may serve a request
-  // without a Verlet list first and one with it later
-  L.vl_cnt = take(two_lists ? sizeof(int) * np : 0);
-  L.vl_idx = take(two_lists ? sizeof(int) * (size_t)kVlCap * np : 0);
-  L.qref = take(two_lists ? sizeof(double) * 3 * np : 0);
+  // (284 bytes a particle; a server's request with a Verlet list takes no
+  // slot that was made for one without, slot_serves)
+  L.vl_cnt = take(P.verlet ? sizeof(int) * np : 0);
+  L.vl_idx = take(P.verlet ? sizeof(int) * (size_t)kVlCap * np : 0);
+  L.qref = take(P.verlet ? sizeof(double) * 3 * np : 0);
   L.vl_flag = take(sizeof(uint64_t) * kVlWords);
   L.bar = take(sizeof(unsigned) * 2);
   L.total = off;
@@ -398,13 +398,15 @@ int slot_alloc(Slot& s, const Params& P, int np_cap, cudaStream_t st) {
   r.start1 = two_lists ? (int*)(base + L.start1) : nullptr;
   r.sorted1 = two_lists ? (int*)(base + L.sorted1) : nullptr;
   r.ws1 = two_lists ? (double*)(base + L.ws1) : nullptr;
-  r.vl_cnt = two_lists ? (int*)(base + L.vl_cnt) : nullptr;
-  r.vl_idx = two_lists ? (int*)(base + L.vl_idx) : nullptr;
-  r.qref = two_lists ? (double*)(base + L.qref) : nullptr;
+  r.vl_cnt = P.verlet ? (int*)(base + L.vl_cnt) : nullptr;
+  r.vl_idx = P.verlet ? (int*)(base + L.vl_idx) : nullptr;
+  r.qref = P.verlet ? (double*)(base + L.qref) : nullptr;
   r.vl_flag = (uint64_t*)(base + L.vl_flag);
   r.bar = (unsigned*)(base + L.bar);  // zeroed with the slot
   return FSL_OK;
 }
+
+bool slot_serves(const Slot& s, const Params& P) { return P.np <= s.np_cap && (!P.verlet || s.r.vl_idx); }
 
 void slot_free(Slot& s) {
   if (s.arena) cudaFree(s.arena);
@@ -471,6 +473,7 @@ int slot_reset_observables(Slot& s, cudaStream_t st) {
 int slot_reset(Slot& s, const Params& P, const double* q, const fsl_config& c, cudaStream_t st) {
   if (!s.arena) return errorf(FSL_E_ARG, "slot not allocated");
   if (P.np > s.np_cap) return errorf(FSL_E_ARG, "%d particles exceed the slot's %d", P.np, s.np_cap);
+  if (!slot_serves(s, P)) return errorf(FSL_E_ARG, "the slot has no room for a Verlet list");
   if (!(class_of(P) == class_of(s.r.P))) return errorf(FSL_E_ARG, "instance is not of the slot's size class");
   if (P.np > 0 && !q) return errorf(FSL_E_ARG, "null positions");
   Rep& r = s.r;

@@ -61,6 +61,9 @@ struct Slot {
 // stays inactive until slot_reset.
 int slot_alloc(Slot& s, const Params& P, int np_cap, cudaStream_t st);
 void slot_free(Slot& s);
+// Whether an allocated slot of P's class has the buffers that P needs: room
+// for its particles and, where its pair forces take one, a Verlet list.
+bool slot_serves(const Slot& s, const Params& P);
 // Puts a new instance (parameters P, positions q on the host) into an
 // allocated slot of its class: positions, LJ table, cleared forces, error
 // word, step counter and bonds.  Enqueued on st.

@@ -94,6 +94,21 @@ int64_t count_slots(const fsl_server* s) {
   return n;
 }
 
+// Frees the idle slot i of class G.  Scheduler thread only.
+void drop_slot(fsl_server* s, SGroup& G, int i) {
+  cudaStreamSynchronize(s->exec.stream);
+  s->bytes_held -= (int64_t)G.slots[i]->bytes;
+  fsl::slot_free(*G.slots[i]);
+  G.slots.erase(G.slots.begin() + i);
+  G.owner.erase(G.owner.begin() + i);
+  // owners of later slots move down one place
+  for (size_t k = i; k < G.owner.size(); ++k)
+    if (G.owner[k]) G.owner[k]->slot = (int)k;
+  G.g.slots.clear();
+  for (auto& sl : G.slots) G.g.slots.push_back(sl.get());
+  G.g.dirty = true;
+}
+
 // Frees idle slots (largest first) until `need` more bytes fit the budget.
 // Scheduler thread only.
 bool make_room(fsl_server* s, int64_t need) {
@@ -111,25 +126,20 @@ bool make_room(fsl_server* s, int64_t need) {
         }
     }
     if (!best) return false;
-    cudaStreamSynchronize(s->exec.stream);
-    s->bytes_held -= (int64_t)best->slots[bi]->bytes;
-    fsl::slot_free(*best->slots[bi]);
-    best->slots.erase(best->slots.begin() + bi);
-    best->owner.erase(best->owner.begin() + bi);
-    // owners of later slots move down one place
-    for (size_t i = bi; i < best->owner.size(); ++i)
-      if (best->owner[i]) best->owner[i]->slot = (int)i;
-    best->g.slots.clear();
-    for (auto& sl : best->slots) best->g.slots.push_back(sl.get());
-    best->g.dirty = true;
+    drop_slot(s, *best, bi);
   }
   return true;
 }
 
-// Puts request r into a slot of its class: a free slot with enough capacity
-// (the smallest such), else a new slot if the budget allows.  Returns 1 if
+// Puts request r into a slot of its class: a free slot that serves it (the
+// smallest such), else a new slot if the budget allows.  Returns 1 if
 // admitted, 0 if it must wait for memory, -1 if it can never fit (r failed).
 int admit(fsl_server* s, Request* r) {
+  const int cap = capacity_for(r->P.np);
+  // Lennard-Jones forces come from the cell list where the whole budget has
+  // no room for a Verlet list
+  if (r->P.verlet && r->P.pair == FSL_PAIR_TABLE_LJ && (int64_t)fsl::slot_bytes(r->P, cap) > s->cfg.hbm_budget)
+    r->P.verlet = r->P.order = 0;
   fsl::ClassKey key = fsl::class_of(r->P);
   auto it = s->groups.find(key);
   if (it == s->groups.end()) {
@@ -142,13 +152,17 @@ int admit(fsl_server* s, Request* r) {
     it = s->groups.emplace(key, std::move(G)).first;
   }
   SGroup& G = *it->second;
-  int pick = -1;
-  for (size_t i = 0; i < G.slots.size(); ++i)
-    if (!G.owner[i] && G.slots[i]->np_cap >= r->P.np &&
-        (pick < 0 || G.slots[i]->np_cap < G.slots[pick]->np_cap))
+  int pick = -1, lacks = -1;  // the slot that serves; one that lacks only the list
+  for (size_t i = 0; i < G.slots.size(); ++i) {
+    if (G.owner[i]) continue;
+    if (!fsl::slot_serves(*G.slots[i], r->P)) {
+      if (r->P.np <= G.slots[i]->np_cap) lacks = (int)i;
+    } else if (pick < 0 || G.slots[i]->bytes < G.slots[pick]->bytes) {
       pick = (int)i;
+    }
+  }
   if (pick < 0) {
-    const int cap = capacity_for(r->P.np);
+    if (lacks >= 0) drop_slot(s, G, lacks);  // the new slot takes its place
     const int64_t need = (int64_t)fsl::slot_bytes(r->P, cap);
     if (need > s->cfg.hbm_budget) {
       r->msg = "request needs more device memory than the server's whole budget";
