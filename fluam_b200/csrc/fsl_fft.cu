@@ -69,7 +69,7 @@ struct FftPlan {
   int line_lw = 0;          // lines per warp
   size_t smem_lines = 0;
   bool use_lines = false;   // the five-pass schedule (picked by fft_autotune)
-  float sched_us[2] = {};   // measured solve transform time: plane, lines
+  float sched_us[2] = {};   // measured solve (W build to velocity): plane, lines
   int plane_pb = 0, plane_threads = 0;      // planes per block, threads per block
   int z_kx = 0, z_ky = 0, z_threads = 0;    // zsolve tile and threads per block
   size_t smem_plane_r = 0, smem_z_r = 0;
@@ -699,11 +699,13 @@ static void reg_transform(const Batch& B, const FftPlan* fp, cudaStream_t s, Pro
 
 // Times the z-pass tile candidates on the class's own spectra (an in-place
 // transform and solve of whatever they hold: the next step rewrites them) and
-// keeps the fastest; then, where the edge has both, the plane schedule
-// against the five-pass one (on the class's W, spectra and velocity buffers,
-// which the step rewrites before reading).  Every candidate computes the
-// same bits, so the choice does not change results.  Once per plan, outside
-// graph capture.
+// keeps the fastest; then, where the edge has both, the solve by the plane
+// schedule against the one by five passes, each with what it needs in a step:
+// the planes build W on the way in, the five passes follow the W build that
+// also clears the field (on the class's W, spectra and velocity buffers,
+// which the step rewrites before reading, and the spread field, which is
+// zero).  Every candidate computes the same bits, so the choice does not
+// change results.  Once per plan, outside graph capture.
 void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
   if (!fp || fp->tuned) return;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -760,15 +762,14 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
     use_pcand(fp, pbest);
     fp->use_lines = lines;
   }
-  if (fp->line_xf[0] && sched_env() == 0) {
-    Prof none;
+  if (fp->line_xf[0] && sched_env() == 0 && !cube_serves(B, fp)) {
     fp->sched_us[0] = fp->sched_us[1] = 1e30f;
     for (int round = 0; round < 3; ++round)
       for (int sc = 0; sc < 2; ++sc) {
         fp->use_lines = sc == 1;
-        reg_transform(B, fp, s, none);  // warm-up
+        launch_solve(B, fp, 1, 1.0, B.tiled, s);  // warm-up
         cudaEventRecord(e0, s);
-        for (int r = 0; r < kTuneReps; ++r) reg_transform(B, fp, s, none);
+        for (int r = 0; r < kTuneReps; ++r) launch_solve(B, fp, 1, 1.0, B.tiled, s);
         cudaEventRecord(e1, s);
         float ms = 0.f;
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) ms = 1e9f;

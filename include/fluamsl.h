@@ -368,8 +368,9 @@ typedef struct fsl_class_tuning {
   int32_t z_threads;             /* threads per block of that tile             */
   int32_t z_candidates;          /* z tiles timed (at most 8)                  */
   float z_us[8];                 /* us per z-pass launch of each candidate     */
-  float schedule_us[2];          /* us per transform: plane, five passes
-                                    (0: not timed)                             */
+  float schedule_us[2];          /* us per solve, from the spread field to the
+                                    velocity: plane, five passes (0: not
+                                    timed)                                     */
   int32_t list_build;            /* 0 separate kernels, 1 one block per
                                     instance, 2 cooperative single launch,
                                     -1 no particles                            */

@@ -233,3 +233,19 @@ def test_class_tuning_reports_picks(fsl):
     t = g.tuning()
     assert t["tuned"] == 1 and t["list_build"] == "cooperative" and t["n"] == 1
     g.close()
+
+
+def test_schedule_times_are_those_of_the_solve(fsl):
+    """The tuner times both schedules with the W build that a step has with
+    them: the plane schedule, whose planes build W, as long as the planes per
+    block that it picked took (without the build it took 0.84 of that here)."""
+    q = uniform_positions(300, (64.0,) * 3, 1)
+    b = fsl.Batch([fsl.make_config((64,) * 3, (64.0,) * 3, kT=0.01, dt=0.01, cutoff=1.5, kernel=3, pair=fsl.PAIR_SOFT, seed=i)
+                   for i in range(40)], [q] * 40)
+    b.step(1)
+    b.sync()
+    t = b.class_tuning()[0]
+    b.close()
+    plane_us, lines_us = t["schedule_us"]
+    assert 0.93 < plane_us / min(t["plane_us"]) < 1.07, t
+    assert lines_us > plane_us
