@@ -49,8 +49,7 @@ struct FftPlan {
   float2 *ex = nullptr, *ey = nullptr, *ez = nullptr;  // exp(+i pi j / m)
   // the whole solve of a small cube in one launch (fsl_fft_cube.cuh), for a
   // single instance; null for other extents
-  void (*cube)(Rep, const float2*, const float*, const float*, const float*, const float2*, const float2*, const float2*,
-               WSrc) = nullptr;
+  void (*cube)(Rep, const float*, const float*, const float*, const float2*, const float2*, const float2*, WSrc) = nullptr;
   int cube_threads = 0;
   size_t smem_cube = 0;
   GPlan* gen = nullptr;  // general passes (fsl_fft_g.cu), where the compiled ones do not serve both parts
@@ -382,10 +381,10 @@ static void pick_z_r(FftPlan* fp) {
   if (fp->nzc == 1) use_zcand(fp, 0);
 }
 
-template <int N, int R, int T>
+template <int N>
 static void pick_cube(FftPlan* fp) {
-  using C = CubeGeom<N, R, T>;
-  fp->cube = k_solve_cube<N, R, T>;
+  using C = CubeGeom<N>;
+  fp->cube = k_solve_cube<N>;
   fp->cube_threads = C::THREADS;
   fp->smem_cube = sizeof(float2) * C::SMEM;
 }
@@ -411,8 +410,8 @@ static void pick_register_kernels(const Params& P, FftPlan* fp) {
   }
   if (P.mx == P.my && P.mx == P.mz) {
     switch (P.mx) {
-      case 16: pick_cube<16, 16, 1>(fp); break;
-      case 24: pick_cube<24, 24, 1>(fp); break;
+      case 16: pick_cube<16>(fp); break;
+      case 24: pick_cube<24>(fp); break;
       default: break;
     }
   }
@@ -642,8 +641,8 @@ static void cube_solve(const Batch& B, const FftPlan* fp, const WSrc& ws, cudaSt
   at[1].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, fp->cube, *B.one, (const float2*)fp->twx, (const float*)fp->sx, (const float*)fp->sy,
-                     (const float*)fp->sz, (const float2*)fp->ex, (const float2*)fp->ey, (const float2*)fp->ez, ws);
+  cudaLaunchKernelEx(&cfg, fp->cube, *B.one, (const float*)fp->sx, (const float*)fp->sy, (const float*)fp->sz, (const float2*)fp->ex,
+                     (const float2*)fp->ey, (const float2*)fp->ez, ws);
 }
 
 // Whether the forward plane pass builds W itself: the plane schedule.

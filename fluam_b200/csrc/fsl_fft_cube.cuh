@@ -17,50 +17,46 @@
 // batch the clusters wait for eight free blocks at a time (256 mixed
 // replicas: 2973 against 2811 us a step).
 //
-// The line transforms, the packing of columns 0 and N/2, the solve and W are
-// the arithmetic of k_plane_fwd_r, k_zsolve_r, k_plane_inv_r (same R x T
-// split) and k_wbuild4: the same bits, alone and in a batch.
+// A line's N points stay in one thread's registers (the N x 1 split of the
+// passes).  The line transforms, the packing of columns 0 and N/2, the solve
+// and W are the arithmetic of k_plane_fwd_r, k_zsolve_r, k_plane_inv_r and
+// k_wbuild4: the same bits, alone and in a batch.
 
 constexpr int kCubeRanks = 8;
 
-template <int N, int RR, int T>
+template <int N>
 struct CubeGeom {
-  using G = LineGeom<RR, T>;
+  using G = LineGeom<N, 1>;
   static constexpr int H = N / 2, MXH = H + 1;
   static constexpr int PPR = 3 * N / kCubeRanks;    // planes per rank
   static constexpr int CPR = MXH * N / kCubeRanks;  // (kx, ky) columns per rank
-  static constexpr int PB = plane_buf<N, RR, T>();
+  static constexpr int PB = plane_buf<N, N, 1>();
   static constexpr int NLZ = 3 * CPR;               // z lines per rank
-  static constexpr int THREADS =
-      ((PPR * H * T > NLZ * T ? PPR * H * T : NLZ * T) + 31) / 32 * 32 < 128
-          ? 128
-          : ((PPR * H * T > NLZ * T ? PPR * H * T : NLZ * T) + 31) / 32 * 32;
-  // float2: twiddles | planes or z lines | half spectrum of the rank's planes
+  static constexpr int LINES = PPR * H > NLZ ? PPR * H : NLZ;
+  static constexpr int THREADS = LINES < 128 ? 128 : (LINES + 31) / 32 * 32;
+  // float2: planes or z lines | half spectrum of the rank's planes
   static constexpr int WORK = PPR * PB > NLZ * G::LS ? PPR * PB : NLZ * G::LS;
-  static constexpr int SMEM = N + WORK + PPR * N * MXH;
+  static constexpr int SMEM = WORK + PPR * N * MXH;
   static_assert(3 * N % kCubeRanks == 0 && MXH * N % kCubeRanks == 0 && N % 4 == 0, "equal shares");
   static_assert(2 * PB >= N * (N + 1), "the real plane fits the line buffer");
 };
 
-template <int N, int RR, int T>
-__global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
-    k_solve_cube(const __grid_constant__ Rep R, const float2* __restrict__ twn, const float* __restrict__ sx, const float* __restrict__ sy,
-                 const float* __restrict__ sz, const float2* __restrict__ ex, const float2* __restrict__ ey,
-                 const float2* __restrict__ ez, const WSrc ws) {
+template <int N>
+__global__ void __launch_bounds__(CubeGeom<N>::THREADS)
+    k_solve_cube(const __grid_constant__ Rep R, const float* __restrict__ sx, const float* __restrict__ sy, const float* __restrict__ sz,
+                 const float2* __restrict__ ex, const float2* __restrict__ ey, const float2* __restrict__ ez, const WSrc ws) {
   fsl_pdl_enter();
   if (!R.active) return;  // (all ranks alike)
   const Params& P = R.P;
   namespace cg = cooperative_groups;
-  using C = CubeGeom<N, RR, T>;
+  using C = CubeGeom<N>;
   using G = typename C::G;
-  constexpr int H = C::H, MXH = C::MXH, PPR = C::PPR, CPR = C::CPR, PB = C::PB, NLZ = C::NLZ, LS = G::LS, TPP = H * T;
+  constexpr int H = C::H, MXH = C::MXH, PPR = C::PPR, CPR = C::CPR, PB = C::PB, NLZ = C::NLZ, LS = G::LS;
   extern __shared__ __align__(16) float2 smem[];
-  float2* stw = smem;
-  float2* work = smem + N;
+  float2* work = smem;
   float2* sp = work + C::WORK;  // [plane][ky][kx]
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)blockIdx.x;
-  for (int i = threadIdx.x; i < N; i += blockDim.x) stw[i] = twn[i];
   // ---- W of the rank's planes, which are consecutive in memory, into real
   // planes of row pitch N + 1
   {
@@ -79,54 +75,34 @@ __global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
           });
   }
   __syncthreads();
-  const int lp = threadIdx.x / TPP, r = threadIdx.x - lp * TPP;
+  const int lp = threadIdx.x / H, c = threadIdx.x - lp * H;  // row pair c, then column c, of plane lp
   const bool on = lp < PPR;
   float2* buf = work + (on ? lp : 0) * PB;
-  const int p = r / T, tx = r - p * T;  // x: row pair p, thread tx of its line
-  const int c = r % H, ty = r / H;      // y: column c, thread ty
-  float2 v[RR];
-  float2 out[G::RT][T];
+  float2 v[N];
   // ---- x forward
   if (on) {
     const float* fw = reinterpret_cast<const float*>(buf);
 #pragma unroll
-    for (int k = 0; k < RR; ++k) {
-      const int x = tx + T * k;
-      v[k] = make_float2(fw[(2 * p) * (N + 1) + x], fw[(2 * p + 1) * (N + 1) + x]);
-    }
+    for (int x = 0; x < N; ++x) v[x] = make_float2(fw[(2 * c) * (N + 1) + x], fw[(2 * c + 1) * (N + 1) + x]);
   }
   __syncthreads();
-  if constexpr (T == 1) {
-    if (on) {
-      RDft<RR>::run(v, -1);
+  if (on) {
+    RDft<N>::run(v, -1);
 #pragma unroll
-      for (int f = 0; f < N; ++f) buf[p * LS + f] = v[f];
-    }
-  } else {
-    if (on) line_fft_a<RR, T>(v, tx, buf + p * LS, stw, -1);
-    __syncthreads();
-    if (on) line_fft_b<RR, T>(buf + p * LS, tx, -1, out);
-    __syncthreads();
-    if (on) {
-#pragma unroll
-      for (int j = 0; j < G::RT; ++j)
-        if (line_has<RR, T>(tx, j))
-#pragma unroll
-          for (int b = 0; b < T; ++b) buf[p * LS + line_freq<RR, T>(tx, j, b)] = out[j][b];
-    }
+    for (int f = 0; f < N; ++f) buf[c * LS + f] = v[f];
   }
   __syncthreads();
   // ---- y forward into the half spectrum
   if (on) {
 #pragma unroll
-    for (int k = 0; k < RR; ++k) {
-      const int y = ty + T * k, q = y >> 1, odd = y & 1;
+    for (int y = 0; y < N; ++y) {
+      const int q = y >> 1, odd = y & 1;
       if (c == 0) {
         const float2 a = buf[q * LS], b = buf[q * LS + H];
-        v[k] = odd ? make_float2(a.y, b.y) : make_float2(a.x, b.x);
+        v[y] = odd ? make_float2(a.y, b.y) : make_float2(a.x, b.x);
       } else {
         const float2 zk = buf[q * LS + c], zm = buf[q * LS + N - c];
-        v[k] = odd ? make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x))
+        v[y] = odd ? make_float2(0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x))
                    : make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
       }
     }
@@ -138,48 +114,19 @@ __global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
     pl[f * MXH] = make_float2(0.5f * (Cf.x + Cm.x), 0.5f * (Cf.y - Cm.y));
     pl[f * MXH + H] = make_float2(0.5f * (Cf.y + Cm.y), -0.5f * (Cf.x - Cm.x));
   };
-  if constexpr (T == 1) {
-    if (on) {
-      RDft<RR>::run(v, -1);
+  if (on) {
+    RDft<N>::run(v, -1);
 #pragma unroll
-      for (int f = 0; f < N; ++f) {
-        if (c != 0) pl[f * MXH + c] = v[f];
-        else unpack(f, v[f], v[(N - f) % N]);
-      }
-    }
-  } else {
-    if (on) line_fft_a<RR, T>(v, ty, buf + c * LS, stw, -1);
-    __syncthreads();
-    if (on) line_fft_b<RR, T>(buf + c * LS, ty, -1, out);
-    __syncthreads();
-    if (on) {
-#pragma unroll
-      for (int j = 0; j < G::RT; ++j)
-        if (line_has<RR, T>(ty, j))
-#pragma unroll
-          for (int b = 0; b < T; ++b) {
-            const int f = line_freq<RR, T>(ty, j, b);
-            if (c != 0) pl[f * MXH + c] = out[j][b];
-            else buf[f] = out[j][b];
-          }
-    }
-    __syncthreads();
-    if (on && c == 0) {
-#pragma unroll
-      for (int j = 0; j < G::RT; ++j)
-        if (line_has<RR, T>(ty, j))
-#pragma unroll
-          for (int b = 0; b < T; ++b) {
-            const int f = line_freq<RR, T>(ty, j, b);
-            unpack(f, out[j][b], buf[(N - f) % N]);
-          }
+    for (int f = 0; f < N; ++f) {
+      if (c != 0) pl[f * MXH + c] = v[f];
+      else unpack(f, v[f], v[(N - f) % N]);
     }
   }
   cl.sync();
   // ---- z lines of the rank's columns, the solve, and back
   {
-    const int l = threadIdx.x % NLZ, t = threadIdx.x / NLZ;
-    const bool zon = t < T;
+    const int l = threadIdx.x % NLZ;
+    const bool zon = threadIdx.x < NLZ;
     const int comp = l / CPR, cc = l - comp * CPR, col = rank * CPR + cc;
     float2* lb = work + l * LS;
     // element z of this line: plane comp N + z of its rank
@@ -189,26 +136,10 @@ __global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
     };
     if (zon) {
 #pragma unroll
-      for (int k = 0; k < RR; ++k) v[k] = *at(t + T * k);
-    }
-    if constexpr (T == 1) {
-      if (zon) {
-        RDft<RR>::run(v, -1);
+      for (int k = 0; k < N; ++k) v[k] = *at(k);
+      RDft<N>::run(v, -1);
 #pragma unroll
-        for (int f = 0; f < N; ++f) lb[f] = v[f];
-      }
-    } else {
-      if (zon) line_fft_a<RR, T>(v, t, lb, stw, -1);
-      __syncthreads();
-      if (zon) line_fft_b<RR, T>(lb, t, -1, out);
-      __syncthreads();
-      if (zon) {
-#pragma unroll
-        for (int j = 0; j < G::RT; ++j)
-          if (line_has<RR, T>(t, j))
-#pragma unroll
-            for (int b = 0; b < T; ++b) lb[line_freq<RR, T>(t, j, b)] = out[j][b];
-      }
+      for (int f = 0; f < N; ++f) lb[f] = v[f];
     }
     __syncthreads();
     {
@@ -247,26 +178,13 @@ __global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
     __syncthreads();
     if (zon) {
 #pragma unroll
-      for (int k = 0; k < RR; ++k) v[k] = lb[t + T * k];
+      for (int k = 0; k < N; ++k) v[k] = lb[k];
     }
     __syncthreads();
-    if constexpr (T == 1) {
-      if (zon) {
-        RDft<RR>::run(v, +1);
+    if (zon) {
+      RDft<N>::run(v, +1);
 #pragma unroll
-        for (int k = 0; k < RR; ++k) *at(k) = v[k];
-      }
-    } else {
-      if (zon) line_fft_a<RR, T>(v, t, lb, stw, +1);
-      __syncthreads();
-      if (zon) {
-        line_fft_b<RR, T>(lb, t, +1, out);
-#pragma unroll
-        for (int j = 0; j < G::RT; ++j)
-          if (line_has<RR, T>(t, j))
-#pragma unroll
-            for (int b = 0; b < T; ++b) *at(line_freq<RR, T>(t, j, b)) = out[j][b];
-      }
+      for (int k = 0; k < N; ++k) *at(k) = v[k];
     }
   }
   cl.sync();  // (no rank touches another's shared memory after this)
@@ -275,13 +193,12 @@ __global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
   static_assert(N * PR <= PB && N * PRF <= 2 * PB, "plane rows fit the plane buffer");
   if (on) {
 #pragma unroll
-    for (int k = 0; k < RR; ++k) {
-      const int ky = ty + T * k;
+    for (int ky = 0; ky < N; ++ky) {
       if (c == 0) {
         const float2 f0 = pl[ky * MXH], fh = pl[ky * MXH + H];
-        v[k] = make_float2(f0.x - fh.y, f0.y + fh.x);  // F0 + i FH
+        v[ky] = make_float2(f0.x - fh.y, f0.y + fh.x);  // F0 + i FH
       } else {
-        v[k] = pl[ky * MXH + c];
+        v[ky] = pl[ky * MXH + c];
       }
     }
   }
@@ -294,70 +211,37 @@ __global__ void __launch_bounds__(CubeGeom<N, RR, T>::THREADS)
       buf[y * PR + c] = u;
     }
   };
-  if constexpr (T == 1) {
-    if (on) {
-      RDft<RR>::run(v, +1);
+  if (on) {
+    RDft<N>::run(v, +1);
 #pragma unroll
-      for (int y = 0; y < N; ++y) put(y, v[y]);
-    }
-  } else {
-    if (on) line_fft_a<RR, T>(v, ty, buf + c * LS, stw, +1);
-    __syncthreads();
-    if (on) line_fft_b<RR, T>(buf + c * LS, ty, +1, out);
-    __syncthreads();
-    if (on) {
-#pragma unroll
-      for (int j = 0; j < G::RT; ++j)
-        if (line_has<RR, T>(ty, j))
-#pragma unroll
-          for (int b = 0; b < T; ++b) put(line_freq<RR, T>(ty, j, b), out[j][b]);
-    }
+    for (int y = 0; y < N; ++y) put(y, v[y]);
   }
   __syncthreads();
   // ---- x inverse
   if (on) {
 #pragma unroll
-    for (int k = 0; k < RR; ++k) {
-      const int x = tx + T * k;
+    for (int x = 0; x < N; ++x) {
       float2 e, o;
       if (x <= H) {
-        e = buf[(2 * p) * PR + x];
-        o = buf[(2 * p + 1) * PR + x];
+        e = buf[(2 * c) * PR + x];
+        o = buf[(2 * c + 1) * PR + x];
       } else {
-        e = buf[(2 * p) * PR + N - x];
-        o = buf[(2 * p + 1) * PR + N - x];
+        e = buf[(2 * c) * PR + N - x];
+        o = buf[(2 * c + 1) * PR + N - x];
         e.y = -e.y;
         o.y = -o.y;
       }
-      v[k] = make_float2(e.x - o.y, e.y + o.x);  // X_2p + i X_2p+1
+      v[x] = make_float2(e.x - o.y, e.y + o.x);  // X_2c + i X_2c+1
     }
   }
   __syncthreads();
   float* fb = reinterpret_cast<float*>(buf);
-  if constexpr (T == 1) {
-    if (on) {
-      RDft<RR>::run(v, +1);
+  if (on) {
+    RDft<N>::run(v, +1);
 #pragma unroll
-      for (int x = 0; x < N; ++x) {
-        fb[(2 * p) * PRF + x] = v[x].x;
-        fb[(2 * p + 1) * PRF + x] = v[x].y;
-      }
-    }
-  } else {
-    if (on) line_fft_a<RR, T>(v, tx, buf + p * LS, stw, +1);
-    __syncthreads();
-    if (on) line_fft_b<RR, T>(buf + p * LS, tx, +1, out);
-    __syncthreads();
-    if (on) {
-#pragma unroll
-      for (int j = 0; j < G::RT; ++j)
-        if (line_has<RR, T>(tx, j))
-#pragma unroll
-          for (int b = 0; b < T; ++b) {
-            const int x = line_freq<RR, T>(tx, j, b);
-            fb[(2 * p) * PRF + x] = out[j][b].x;
-            fb[(2 * p + 1) * PRF + x] = out[j][b].y;
-          }
+    for (int x = 0; x < N; ++x) {
+      fb[(2 * c) * PRF + x] = v[x].x;
+      fb[(2 * c + 1) * PRF + x] = v[x].y;
     }
   }
   __syncthreads();
