@@ -85,6 +85,72 @@ def test_step_io_then_plain_steps(fsl):
     b.close()
 
 
+def _follow(fsl, cfg, q0):
+    """step_io on a pinned buffer against set_positions, step and positions,
+    with host moves in between (2-D instances: in the plane)."""
+    import torch
+    a, b = fsl.StokesLimit(cfg, q0), fsl.StokesLimit(cfg, q0)
+    buf = torch.empty(q0.shape, dtype=torch.float64).pin_memory()
+    qa = buf.numpy()
+    qa[...] = q0
+    rng = np.random.default_rng(12)
+    for k in range(5):
+        qb = qa.copy()
+        a.step_io(qa, qa)
+        b.set_positions(qb)
+        b.step(1)
+        yield qa, b.positions()
+        qa[:2] += rng.normal(0.0, 0.01, (2, q0.shape[1]))
+        if k % 2:
+            idx = rng.choice(q0.shape[1], 20, replace=False)
+            qa[:2, idx] += rng.normal(0.0, 0.5, (2, 20))
+    sa = a.status()
+    assert sa["step"] == 5 and sa["error_bits"] == 0 and sa["graph"]
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("n", [16384, 16385])
+def test_step_io_kernels_and_copy_nodes(fsl, n):
+    """Page-locked buffers up to 16,384 particles by kernels, from there on
+    by copy nodes and the moved check in the step's graph."""
+    for got, want in _follow(fsl, _config(fsl), uniform_positions(n, (48, 48, 48), 7)):
+        np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("n", [300, 17000])
+@pytest.mark.parametrize("scheme", ["SCHEME_FIRST_ORDER", "SCHEME_QUASI2D", "SCHEME_STOKES2D"])
+def test_step_io_other_schemes(fsl, scheme, n):
+    two_d = scheme != "SCHEME_FIRST_ORDER"
+    m = (48, 48, 1) if two_d else (48, 48, 48)
+    L = (48.0, 48.0, 4.0) if two_d else (48.0,) * 3
+    q0 = uniform_positions(n, L, 8)
+    if two_d:
+        q0[2] = 0.0
+    cfg = fsl.make_config(m, L, kT=0.01, dt=0.01, cutoff=1.5, kernel=3, pair=fsl.PAIR_SOFT, seed=42, radius=1.0,
+                          extra_mobility=0.0 if two_d else 0.2, scheme=getattr(fsl, scheme))
+    for got, want in _follow(fsl, cfg, q0):
+        if two_d:  # FP64 atomics: sums in any order, rounding of a thousand terms
+            np.testing.assert_allclose(got, want, rtol=0, atol=1e-11 * 48)
+        else:
+            np.testing.assert_array_equal(got, want)
+
+
+def test_step_io_without_particles(fsl):
+    """The incompressible fluid has no positions: the step alone."""
+    import torch
+    cfg = fsl.make_config((16, 16, 16), (16.0,) * 3, kT=0.01, dt=0.05, seed=3, scheme=fsl.SCHEME_INCOMPRESSIBLE)
+    a, b = fsl.StokesLimit(cfg, np.zeros((3, 0))), fsl.StokesLimit(cfg, np.zeros((3, 0)))
+    buf = torch.empty(8, dtype=torch.float64).pin_memory()
+    for _ in range(3):
+        a.step_io(buf.data_ptr(), buf.data_ptr())
+    b.step(3)
+    np.testing.assert_array_equal(a.velocity64(), b.velocity64())
+    assert a.status()["step"] == 3
+    a.close()
+    b.close()
+
+
 def test_step_io_unaligned_buffer(fsl):
     """Page-locked doubles at an address that is no multiple of 8 (or of 4):
     taken by copies, which have no alignment."""
