@@ -331,6 +331,8 @@ int fsl_set_step(fsl_handle* h, uint64_t step) {
   if (!h) return errorf(FSL_E_ARG, "null handle");
   FSL_TRY(cudaSetDevice(h->exec.device));
   FSL_TRY(cudaMemcpyAsync(rep(h).t, &step, sizeof(step), cudaMemcpyHostToDevice, h->exec.stream));
+  // a rebuild of the Verlet list is asked for by the step it is due in
+  if (int rc = fsl::slot_mark_moved(h->slot, h->exec.stream)) return rc;
   FSL_TRY(cudaStreamSynchronize(h->exec.stream));
   return FSL_OK;
 }

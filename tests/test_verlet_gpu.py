@@ -106,6 +106,21 @@ def test_verlet_after_set_positions_and_entry_points(fsl):
         np.testing.assert_allclose(b.positions(), a.positions(), rtol=0, atol=1e-12)
 
 
+def test_verlet_rebuild_survives_set_step(fsl):
+    """Particles cross the skin in nearly every step; a counter set in between
+    does not lose the rebuild that the last update asked for."""
+    q = uniform_positions(4000, (32.0,) * 3, 5)
+    a, b = _pair(fsl, q, dt=2.0)
+    with a, b:
+        for k in range(6):
+            for x in (a, b):
+                x.step(1)
+                x.set_step(1000 - 50 * k)
+            qa, qb = a.positions(), b.positions()
+            assert np.abs(qa - qb).max() <= 1e-9 * np.abs(qa - q).max(), k
+        assert np.abs(qa - q).max() > 0.4
+
+
 def test_verlet_overflow_falls_back_to_cells(fsl):
     """More than 64 neighbours within rc + skin (a dense random box, as the
     served workload draws): the instance switches to the cell-list pair
