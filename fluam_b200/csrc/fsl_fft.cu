@@ -763,7 +763,7 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
   }
   if (fp->line_xf[0] && sched_env() == 0 && !cube_serves(B, fp)) {
     fp->sched_us[0] = fp->sched_us[1] = 1e30f;
-    for (int round = 0; round < 3; ++round)
+    for (int round = 0; round < 3; ++round) {
       for (int sc = 0; sc < 2; ++sc) {
         fp->use_lines = sc == 1;
         launch_solve(B, fp, 1, 1.0, B.tiled, s);  // warm-up
@@ -774,6 +774,10 @@ void fft_autotune(FftPlan* fp, const Batch& B, cudaStream_t s) {
         if (cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess) ms = 1e9f;
         fp->sched_us[sc] = std::min(fp->sched_us[sc], ms * 1000.f / kTuneReps);
       }
+      // a first round that is far from even settles it (the passes are warm
+      // by now): 128^3 alone 0.8 ms instead of 2.4
+      if (std::max(fp->sched_us[0], fp->sched_us[1]) > 1.2f * std::min(fp->sched_us[0], fp->sched_us[1])) break;
+    }
     fp->use_lines = fp->sched_us[1] < fp->sched_us[0];
   }
   cudaEventDestroy(e0);
