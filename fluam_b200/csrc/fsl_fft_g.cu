@@ -798,9 +798,13 @@ bool g_build(GPlan* g, int optin) {
   const int es = (int)sizeof(V), bank = es == 8 ? 16 : 8;
   const GAxis &ax = g->ax, &ay = g->ay, &az = g->az;
   const int npairs = (g->my + 1) / 2;
-  // ---- whole planes: both extents in two stages, at least four blocks of
-  // 256 threads' worth of shared memory is not asked for: a plane that fits
-  // at all saves a pass of the spectrum through the L2 or HBM
+  // ---- whole planes, where both extents have two stages and a plane fits:
+  // that saves a pass of the spectrum through the L2 or HBM (60 x 72 x 100,
+  // 300 planes: 25 us a solve).  A quasi-2D field has two planes, so two
+  // blocks do the work, which is the faster way up to about 80^2 only: a step
+  // by planes and by one-axis passes 40 and 48 us at 32^2, 44 and 50 at 64^2,
+  // 66 and 58 at 96^2, 72 and 58 at 128^2, 89 and 64 at 144^2; the rule does
+  // not tell them apart yet.
   if (ax.ns == 2 && ay.ns == 2) {
     g->p_rmax = std::max(g_rmax(ax), g_rmax(ay));
     const int cap = g_nt<V>(g->p_rmax);

@@ -253,13 +253,16 @@ int make_params(const fsl_config& c, int64_t np, Params& P) {
   // within two cells), no list at all without pair forces.  The table of the
   // Lennard-Jones force is exactly zero from rc on, so pairs beyond rc on the
   // list add nothing; its cutoffs are several particles wide, so its skin is
-  // smaller, and a density that would often fill the kVlCap slots keeps it on
-  // the cell-list kernel: beyond 40 expected neighbours, 24 of which (3.8
-  // standard deviations of a uniform density) are left to chance.  A list
-  // that overflows all the same, or that particles outrun, gives way to the
-  // cell list (vl_no_build).  At 64^3 cells, 8,000 particles, rc = 5 the
-  // cell list, rebuilt for each evaluation, and its force kernel took 83 of
-  // 238 us of a step's kernels.
+  // smaller (64^3, rc = 5, us a step with rc/16, rc/8 and rc/4: 9,261 slow
+  // particles 114, 114 and 114, faster ones, kT = 0.1, 179, 114 and 114,
+  // faster still 189, 184 and 115; 96^3 with 37 neighbours 273, 279 and 317;
+  // a dense half box 126, 133 and, overflowing, 218), and a density that would
+  // often fill the kVlCap slots keeps it on the cell-list kernel: beyond 40
+  // expected neighbours, the other 24 slots being 3.8 standard deviations of a
+  // uniform density.  A list that overflows all the same, or that particles
+  // outrun, gives way to the cell list (vl_no_build).  At 64^3 cells, 8,000
+  // particles, rc = 5 the cell list, rebuilt for each evaluation, and its
+  // force kernel took 83 of 238 us of a step's kernels.
   // FLUAMSL_VERLET=0 keeps pair forces on the cell-list kernel.
   if (c.scheme <= FSL_SCHEME_FIRST_ORDER && np > 0) {
     const bool pairs_on = c.nonbonded && c.pair != FSL_PAIR_NONE;
